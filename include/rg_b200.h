@@ -210,7 +210,8 @@ int32_t rg_b200_prefill(rg_session *s, int32_t row, const int32_t *ids, size_t n
  * rows must be distinct.  Chunks of up to 1024 columns are cut across the prompts, so short prompts
  * share every weight tile.  last_logits (nullable) receives [n_rows, vocab], the logits after each
  * prompt's last token; greedy (nullable) the token selected from them.  Everything is validated
- * before any device work, and no row's position advances unless the whole call succeeded. */
+ * before any device work, and no row's position advances unless the whole call succeeded.  In chunks of more than 32
+ * columns a prompt's cache rows are the same bits whatever shares the chunk; smaller chunks add up in another order. */
 int32_t rg_b200_prefill_rows(rg_session *s, const int32_t *rows, const int32_t *ids, const size_t *lens, int32_t n_rows,
                              float *last_logits, int32_t *greedy);
 /* run_token (metal_generation.rs:1123-1138) generalised to `batch` rows (batch.rs:140-162):

@@ -154,9 +154,8 @@ cudaError_t launch_qgemm_tc(const QGemmArgs &a, const LaunchCfg &cfg);
 // 128 x 512 tiles with the A operand in shared memory (qgemm_tc_wide.cu): single-operand modes, Q4_0, m > 256
 bool qgemm_tc_wide_applies(const QGemmArgs &a);
 cudaError_t launch_qgemm_tc_wide(const QGemmArgs &a, const LaunchCfg &cfg);
-int qgemm_effective_splits(int k, int splits);
-int qgemm_rows_per_cta(int mode);
-int qgemm_auto_splits(int n, int k, int m, int mode, int sm_count, size_t scratch_floats);
+constexpr int QGEMM_SPLIT_MAX_TOKENS = 32;  // products of more tokens add up all of K in one fixed order
+int qgemm_splits(int n, int k, int m, int mode, int sm_count, size_t scratch_floats);
 // out[r][i] (+)= sum over s < splits of part[s * stride + r * n + i]
 cudaError_t launch_reduce_splits(const float *part, int splits, size_t stride, int n, int rows, float *out, int ldo, bool accumulate,
                                  const LaunchCfg &cfg);

@@ -675,40 +675,25 @@ cudaError_t launch_reduce_splits(const float *part, int splits, size_t stride, i
                        dim3((unsigned)((n + 255) / 256), (unsigned)rows), dim3(256), cfg, part, splits, stride, n, out, ldo);
 }
 
-// K splits of a GEMM of m tokens.  A CTA covers 256 (128) weight rows and 128 (256) tokens, so that few rows or few tokens
-// leave most SMs idle (16 of 148 CTAs for [4096, 4096] with up to 128 tokens), and a nearly empty last wave costs as
-// much as a full one.  The count that gives the fewest raw tiles (256 columns) per SM wins; a wave is charged a quarter
-// of a raw tile for its start, and the partial sums, written and read back through L2, one raw tile (6 us in the
-// compensated mode) per 24 MB.  117 tokens on the 8B shape: a prompt takes 9.1 ms where unsplit products took 22.3 ms
-// (q|k|v 6 splits, O and down 8, gate|up, whose 112 CTAs nearly fill the GPU, none); at 1024 tokens nothing is split.
-int qgemm_auto_splits(int n, int k, int m, int mode, int sm_count, size_t scratch_floats) {
-  const int rows = qgemm_rows_per_cta(mode), toks = mode == QGEMM_F16X3 ? 128 : 256;
-  const long tiles = (long)((n + rows - 1) / rows) * ((m + toks - 1) / toks);
+// Number of K splits a launch with these arguments will actually use (whole 256-column raw tiles each).
+static int effective_splits(int k, int splits) {
   const int raws = k / (KSTEP * RAW_STEPS);
-  int best = 1;
-  double best_cost = (double)((tiles + sm_count - 1) / sm_count) * raws;
-  for (int want = 2; want <= raws && want * tiles <= 8L * sm_count; ++want) {
-    const int s = qgemm_effective_splits(k, want);
-    if (s != want || (size_t)s * (size_t)m * (size_t)n > scratch_floats) continue;
-    const double bytes = 8.0 * s * (double)m * (double)n;
-    const double cost = (double)((tiles * s + sm_count - 1) / sm_count) * ((raws + s - 1) / s + 0.25) + bytes / 24e6;
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = s;
-    }
-  }
-  return best;
+  if (splits < 1) splits = 1;
+  const int per_split = (raws + splits - 1) / splits;
+  return (raws + per_split - 1) / per_split;
 }
 
-// Weight rows one CTA covers in this operand mode.
-int qgemm_rows_per_cta(int mode) { return TM * row_tiles(mode); }
-
-// Number of K splits a launch with these arguments will actually use (whole 256-column raw tiles each).
-int qgemm_effective_splits(int k, int splits) {
-  const int total_steps = k / KSTEP;
-  if (splits < 1) splits = 1;
-  const int k_steps = ((total_steps / RAW_STEPS + splits - 1) / splits) * RAW_STEPS;
-  return (total_steps + k_steps - 1) / k_steps;
+// K splits of a GEMM of m tokens.  Up to 32 tokens (one token tile) a projection of 4096 rows has 16 CTAs for 148 SMs and
+// streams weights, so K is cut until about two CTAs per SM exist.  The count follows from the weight's shape, not from
+// m (a scratch too small for the partial tiles lowers it).  Above 32 tokens K stays whole: a count that follows the
+// tokens would make a prompt's sums, and through its f16 cache rows its later ids, depend on the prompts that share its
+// chunk.
+int qgemm_splits(int n, int k, int m, int mode, int sm_count, size_t scratch_floats) {
+  if (m > QGEMM_SPLIT_MAX_TOKENS || k < KSTEP * RAW_STEPS) return 1;
+  const int rows = TM * row_tiles(mode), tiles = (n + rows - 1) / rows;
+  int splits = effective_splits(k, 2 * sm_count / tiles);
+  while (splits > 1 && (size_t)splits * (size_t)m * (size_t)n > scratch_floats) --splits;
+  return effective_splits(k, splits);  // the launcher's own count: the reduction sums exactly the tiles it writes
 }
 
 cudaError_t launch_qgemm_tc(const QGemmArgs &a, const LaunchCfg &cfg) {

@@ -923,7 +923,7 @@ static int32_t gemm_tc(rg_session *s, const DevTensor &w, int m, float *out, int
   a.out = out;
   a.ldc = ldc;
   prof_mark(s, PROF_GEMV);
-  const int splits = qgemm_auto_splits(a.n, a.k, m, s->gemm_mode, s->sm_count, s->split_scratch_floats);
+  const int splits = qgemm_splits(a.n, a.k, m, s->gemm_mode, s->sm_count, s->split_scratch_floats);
   if (splits > 1) {
     a.accumulate = false;  // the reduction adds
     a.out = s->split_scratch;
@@ -1931,8 +1931,8 @@ int32_t rg_b200_session_prepare(rg_plan *p, rg_session **out) {
   uint8_t *raw;
   s->xb_ld = std::max(d, std::max(qw, s->ffn_l));
   RG_TRY(dalloc(s.get(), &raw, (size_t)2 * WMAX * s->xb_ld * 2));
-  // two partial tiles of 256 rows x 128 tokens per SM (39 MB); the weight-streaming products need less
-  s->split_scratch_floats = (size_t)2 * s->sm_count * 256 * 128;
+  // two partial tiles of 256 rows x 32 tokens per SM (9.7 MB)
+  s->split_scratch_floats = (size_t)2 * s->sm_count * 256 * QGEMM_SPLIT_MAX_TOKENS;
   RG_TRY(dalloc(s.get(), &s->split_scratch, s->split_scratch_floats));
   RG_TRY(dalloc(s.get(), &s->ssq_a, (size_t)256 * 16));
   RG_TRY(dalloc(s.get(), &s->ssq_b, (size_t)256 * 16));
