@@ -959,7 +959,10 @@ static int32_t forward_wide(rg_session *s, int ncols, int n_logit_cols, bool adv
     prof_mark(s, PROF_OTHER);
     RG_LAUNCH(s, launch_rmsnorm16(s->x, d, reinterpret_cast<const float *>(W.attn_norm.d), d, c.norm_eps, ncols, xop,
                                   (tp_lib && l > 0) ? plain : L));
-    if (W.qkv_stacked) {  // one GEMM over the stacked rows of q | k | v
+    // one GEMM over the stacked rows of q | k | v where K is not split: a split's part count follows from the rows of one
+    // matrix, so the sums stay those of separate products
+    const bool whole_k = ncols > QGEMM_SPLIT_MAX_TOKENS;
+    if (W.qkv_stacked && whole_k) {
       DevTensor all = W.q;
       all.rows = W.q.rows + W.k.rows + W.v.rows;
       all.nbytes = W.q.nbytes + W.k.nbytes + W.v.nbytes;
@@ -1078,7 +1081,7 @@ static int32_t forward_wide(rg_session *s, int ncols, int n_logit_cols, bool adv
     prof_mark(s, PROF_OTHER);
     RG_LAUNCH(s, launch_rmsnorm16(s->x, d, reinterpret_cast<const float *>(W.ffn_norm.d), d, c.norm_eps, ncols, xop,
                                   tp_lib ? plain : L));
-    if (W.gu_stacked) {  // one GEMM over gate | up: token rows of [gate, up] side by side
+    if (W.gu_stacked && whole_k) {  // one GEMM over gate | up: token rows of [gate, up] side by side
       DevTensor all = W.gate;
       all.rows = W.gate.rows + W.up.rows;
       all.nbytes = W.gate.nbytes + W.up.nbytes;

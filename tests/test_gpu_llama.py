@@ -846,3 +846,21 @@ def test_a_prompt_leaves_the_same_cache_rows_whatever_shares_its_chunk(n, kv_f32
         fill()
         behind.append(s.run_token(7))
     assert np.array_equal(behind[1], behind[0]) and np.array_equal(behind[2], behind[0])
+
+
+@pytest.mark.parametrize("n", [9, 16, 17, 32, 33, 64, 300])
+@pytest.mark.parametrize("body", [quant.Q4_0, quant.Q8_0], ids=["q4_0", "q8_0"])
+def test_stacked_projections_give_the_sums_of_separate_ones(n, body, monkeypatch):
+    """q | k | v and gate | up in one allocation, multiplied as one product or as separate ones, give the same bits at
+    every chunk size: where K is split (up to 32 columns) the number of parts follows from the rows of each matrix,
+    and here gate and up together (78 row tiles) would be cut into 3 parts, each by itself (39) into 4."""
+    cfg = synth.scaled(synth.TINY, d_model=2048, n_heads=16, n_kv_heads=4, head_dim=128, ffn_dim=9984, vocab=640, n_layers=2,
+                       rope_theta=500000.0, max_context=320)
+    prompt = synth.prompt_ids(cfg, n, seed=n)
+    got = []
+    for stacked in (True, False):
+        monkeypatch.setenv("RG_B200_NO_STACKED_GEMM", "0" if stacked else "1")
+        target = session.CudaSessionTarget(max_context=320)
+        s = session.LlamaCudaPlan.synthetic(cfg, target, seed=5, body_type=body).prepare()
+        got.append((s.prefill_ids(prompt), s.run_token(7)))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
