@@ -1066,17 +1066,11 @@ static int32_t forward_wide(rg_session *s, int ncols, int n_logit_cols, bool adv
     }
     }
     if (!attn_in_operand) RG_LAUNCH(s, launch_to16(s->attn_f32, qw, qw, ncols, xop, L));
-    const bool add_in_gemm = !tp;  // one GPU: the projection adds into the residual stream itself
-    if (add_in_gemm) {
-      if ((rc = gemm_tc(s, W.o, ncols, s->x, d, L, true))) return rc;
-    } else {
+    if (tp) {
       if ((rc = gemm_tc(s, W.o, ncols, s->tp_part[0], d, L))) return rc;
-      if (tp) {
-        if ((rc = tp_reduce_add(s, ncols, 0))) return rc;
-      } else {
-        prof_mark(s, PROF_OTHER);
-        RG_LAUNCH(s, launch_add_rows(s->x, d, s->tp_part[0], d, d, ncols, L));
-      }
+      if ((rc = tp_reduce_add(s, ncols, 0))) return rc;
+    } else {  // one GPU: the projection adds into the residual stream itself
+      if ((rc = gemm_tc(s, W.o, ncols, s->x, d, L, true))) return rc;
     }
     prof_mark(s, PROF_OTHER);
     RG_LAUNCH(s, launch_rmsnorm16(s->x, d, reinterpret_cast<const float *>(W.ffn_norm.d), d, c.norm_eps, ncols, xop,
@@ -1094,16 +1088,11 @@ static int32_t forward_wide(rg_session *s, int ncols, int n_logit_cols, bool adv
       prof_mark(s, PROF_OTHER);
       RG_LAUNCH(s, launch_swiglu16(s->gate_f32, s->up_f32, s->ffn_l, s->ffn_l, ncols, xop, L));
     }
-    if (add_in_gemm) {
-      if ((rc = gemm_tc(s, W.down, ncols, s->x, d, L, true))) return rc;
-    } else {
+    if (tp) {
       if ((rc = gemm_tc(s, W.down, ncols, s->tp_part[1], d, L))) return rc;
-      if (tp) {
-        if ((rc = tp_reduce_add(s, ncols, 1))) return rc;
-      } else {
-        prof_mark(s, PROF_OTHER);
-        RG_LAUNCH(s, launch_add_rows(s->x, d, s->tp_part[1], d, d, ncols, L));
-      }
+      if ((rc = tp_reduce_add(s, ncols, 1))) return rc;
+    } else {
+      if ((rc = gemm_tc(s, W.down, ncols, s->x, d, L, true))) return rc;
     }
   }
   if (n_logit_cols > 0) {
