@@ -22,7 +22,12 @@ constexpr int KSTEP = 64;     // elements per stage (128 bytes: one swizzle row)
 constexpr int RAW_STEPS = 4;  // 64-element stages per raw weight tile (256 columns = 8 blocks)
 constexpr int RAW_NS = 2;     // raw ring depth
 constexpr int THREADS = 320;  // TMA warp, MMA warp, eight dequantisation / epilogue warps
-constexpr int A_BYTES = TM * KSTEP * 2;
+constexpr int TN = 512;       // tokens per tile: two 256-column accumulators
+constexpr int NS = 2;         // operand ring depth
+constexpr int A_BYTES = TM * KSTEP * 2, B_BYTES = TN * KSTEP * 2;  // one stage of each operand
+constexpr int BB = 18;           // bytes of a Q4_0 block
+constexpr int RAW_ROW = 8 * BB;  // bytes of one weight row in a raw tile
+constexpr int RAW_BYTES = TM * RAW_ROW;
 
 struct Params {
   int n, k;     // weight rows, columns
@@ -135,45 +140,15 @@ __device__ __forceinline__ void q4_block_to_16(uint32_t dbits16, const uint32_t 
     out[8 + 2 * i + 1] = mul2<F16>(sub2<F16>(((w >> 12) & M) | E, OFF), d2);
   }
 }
-// One Q8_0 block (eight words of int8) -> 32 values.
+
 template <bool F16>
-__device__ __forceinline__ void q8_block_to_16(uint32_t dbits16, const uint32_t (&q)[8], uint32_t (&out)[16]) {
-  const float d = half_bits_to_float(dbits16);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t u = q[i] ^ 0x80808080u;
-    const float v0 = __uint_as_float(0x4B000000u | (u & 0xffu)) - 8388736.0f;
-    const float v1 = __uint_as_float(0x4B000000u | ((u >> 8) & 0xffu)) - 8388736.0f;
-    const float v2 = __uint_as_float(0x4B000000u | ((u >> 16) & 0xffu)) - 8388736.0f;
-    const float v3 = __uint_as_float(0x4B000000u | (u >> 24)) - 8388736.0f;
-    out[2 * i] = pack2<F16>(v0 * d, v1 * d);
-    out[2 * i + 1] = pack2<F16>(v2 * d, v3 * d);
-  }
-}
-
-__host__ __device__ constexpr int ring_depth(int tn, bool comp) {
-  return comp ? (tn >= 128 ? 2 : 3) : (tn > 256 ? 2 : tn > 128 ? 3 : 4);
-}
-
-template <int QT, int TN, int MODE>
 __global__ void __launch_bounds__(THREADS, 1)
-    qgemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap xlo_map,
-                    const __grid_constant__ CUtensorMap wmap, const Params P) {
-  constexpr bool Q4 = (QT == RG_TYPE_Q4_0);
-  constexpr bool F16 = MODE != QGEMM_BF16, COMP = MODE == QGEMM_F16X3;
-  constexpr int NPL = COMP ? 2 : 1;  // operand planes per stage: hi (and lo)
-  constexpr int BB = Q4 ? 18 : 34;
-  constexpr int NS = ring_depth(TN, COMP);  // operand ring depth
-  constexpr int B_BYTES = TN * KSTEP * 2;
-  constexpr int A_STAGE = NPL * A_BYTES, B_STAGE = NPL * B_BYTES;
-  constexpr int RAW_ROW = 8 * BB;  // bytes of one weight row in a raw tile (144 / 272)
-  constexpr int RAW_BYTES = TM * RAW_ROW;
-  constexpr int TMEM_COLS = TN < 32 ? 32 : TN;
+    qgemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const Params P) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t *a_ring = smem;
-  uint8_t *b_ring = smem + NS * A_STAGE;
-  uint8_t *raw_ring = b_ring + NS * B_STAGE;
+  uint8_t *b_ring = smem + NS * A_BYTES;
+  uint8_t *raw_ring = b_ring + NS * B_BYTES;
   uint64_t *bars = reinterpret_cast<uint64_t *>(raw_ring + RAW_NS * RAW_BYTES);
   uint64_t *b_full = bars, *a_full = bars + NS, *slot_free = bars + 2 * NS;
   uint64_t *raw_full = bars + 3 * NS, *raw_free = raw_full + RAW_NS, *acc_done = raw_free + RAW_NS;
@@ -200,7 +175,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     mbar_fence_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TN)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -224,11 +199,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
         const int slot = i % NS;
         if (i >= NS) mbar_wait_bounded(&slot_free[slot], (uint32_t)((i / NS - 1) & 1), dead, P.status);
-        mbar_expect_tx(&b_full[slot], (uint32_t)B_STAGE);
-        tma_tile_2d(b_ring + slot * B_STAGE, &xmap, (step0 + i) * KSTEP, tok0, &b_full[slot]);
-        if constexpr (TN > 256)  // a TMA box holds at most 256 rows: the second half of the token tile
-          tma_tile_2d(b_ring + slot * B_STAGE + 256 * 128, &xmap, (step0 + i) * KSTEP, tok0 + 256, &b_full[slot]);
-        if constexpr (COMP) tma_tile_2d(b_ring + slot * B_STAGE + B_BYTES, &xlo_map, (step0 + i) * KSTEP, tok0, &b_full[slot]);
+        mbar_expect_tx(&b_full[slot], (uint32_t)B_BYTES);
+        tma_tile_2d(b_ring + slot * B_BYTES, &xmap, (step0 + i) * KSTEP, tok0, &b_full[slot]);
+        // a TMA box holds at most 256 rows: the second half of the token tile
+        tma_tile_2d(b_ring + slot * B_BYTES + 256 * 128, &xmap, (step0 + i) * KSTEP, tok0 + 256, &b_full[slot]);
       }
     }
   } else if (warp == 1) {
@@ -240,28 +214,20 @@ __global__ void __launch_bounds__(THREADS, 1)
       const uint64_t b_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(b_ring), 0));
       const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
       // a 512-token tile is two 256-column accumulators fed by the same dequantised A tile
-      constexpr int MMA_N = TN > 256 ? 256 : TN;
-      constexpr uint32_t idesc = umma_idesc(TM, MMA_N, F16);
+      constexpr uint32_t idesc = umma_idesc(TM, TN / 2, F16);
       for (int i = 0; i < nsteps; ++i) {
         const int slot = i % NS;
         const uint32_t ph = (uint32_t)((i / NS) & 1);
         mbar_wait_bounded(&a_full[slot], ph, dead, P.status);
         mbar_wait_bounded(&b_full[slot], ph, dead, P.status);
         tc_fence_after();
-        const uint64_t a_desc = a_desc0 + (uint64_t)((slot * A_STAGE) >> 4), b_desc = b_desc0 + (uint64_t)((slot * B_STAGE) >> 4);
+        const uint64_t a_desc = a_desc0 + (uint64_t)((slot * A_BYTES) >> 4), b_desc = b_desc0 + (uint64_t)((slot * B_BYTES) >> 4);
         if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < KSTEP / 16; ++kk) {
           const uint64_t a_hi = a_desc + (uint64_t)(kk * 2), b_hi = b_desc + (uint64_t)(kk * 2);
-          if constexpr (COMP) {  // the small terms first, then hi.hi
-            umma_16bit(tmem_u, a_hi, b_hi + (uint64_t)(B_BYTES >> 4), idesc, (i > 0 || kk > 0) ? 1u : 0u);
-            umma_16bit(tmem_u, a_hi + (uint64_t)(A_BYTES >> 4), b_hi, idesc, 1u);
-            umma_16bit(tmem_u, a_hi, b_hi, idesc, 1u);
-          } else {
-            umma_16bit(tmem_u, a_hi, b_hi, idesc, (i > 0 || kk > 0) ? 1u : 0u);
-            if constexpr (TN > 256)
-              umma_16bit(tmem_u + 256, a_hi, b_hi + (uint64_t)((256 * 128) >> 4), idesc, (i > 0 || kk > 0) ? 1u : 0u);
-          }
+          umma_16bit(tmem_u, a_hi, b_hi, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+          umma_16bit(tmem_u + 256, a_hi, b_hi + (uint64_t)((256 * 128) >> 4), idesc, (i > 0 || kk > 0) ? 1u : 0u);
         }
         umma_commit(&slot_free[slot]);  // the slot may be rewritten once these MMAs have read it
         }
@@ -274,7 +240,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     // stage's 64 columns) of one weight row per thread, two threads per row
     const int tdq = threadIdx.x - 64;          // 0..255
     const int r = tdq & 127, half = tdq >> 7;  // row of the tile, even / odd block of the stage
-    constexpr int QW = Q4 ? 4 : 8;             // quant words per block
+    constexpr int QW = 4;                      // quant words per block
     for (int i = 0; i < nsteps; ++i) {
       const int slot = i % NS;
       const int j = i / RAW_STEPS, rs = j % RAW_NS, sub = i % RAW_STEPS;
@@ -295,24 +261,14 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
         for (int w = 0; w < QW; ++w) q[w] = src[QW + 1 + w];
       }
-      uint32_t lows[1];
-      static_assert(!COMP, "the compensated mode runs in qgemm_tc.cu");
-      if constexpr (Q4) {
-        q4_block_to_16<F16>(dbits, q, vals);
-      } else {
-        q8_block_to_16<F16>(dbits, q, vals);
-      }
+      q4_block_to_16<F16>(dbits, q, vals);
       if (sub == RAW_STEPS - 1 || i + 1 == nsteps) mbar_arrive(&raw_free[rs]);  // raw bytes are in registers now
       if (i >= NS) mbar_wait_bounded(&slot_free[slot], (uint32_t)((i / NS - 1) & 1), dead, P.status);
-      uint8_t *row_dst = a_ring + slot * A_STAGE + r * 128;
+      uint8_t *row_dst = a_ring + slot * A_BYTES + r * 128;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint4 chunk = make_uint4(vals[4 * c], vals[4 * c + 1], vals[4 * c + 2], vals[4 * c + 3]);
+        const uint4 chunk = make_uint4(vals[4 * c], vals[4 * c + 1], vals[4 * c + 2], vals[4 * c + 3]);
         *reinterpret_cast<uint4 *>(row_dst + (((4 * half + c) ^ (r & 7)) << 4)) = chunk;
-        if constexpr (COMP) {
-          chunk = make_uint4(lows[4 * c], lows[4 * c + 1], lows[4 * c + 2], lows[4 * c + 3]);
-          *reinterpret_cast<uint4 *>(row_dst + A_BYTES + (((4 * half + c) ^ (r & 7)) << 4)) = chunk;
-        }
       }
       proxy_fence_async();  // generic-proxy stores must be visible to the tensor core's async reads
       mbar_arrive(&a_full[slot]);
@@ -350,7 +306,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TN) : "memory");
   }
 }
 
@@ -369,27 +325,21 @@ EncodeFn encode_fn() {
   return fn;
 }
 
-template <int QT, int TN, int MODE>
+template <bool F16>
 cudaError_t launch_t(const QGemmArgs &a, const LaunchCfg &cfg) {
   EncodeFn fn = encode_fn();
   if (!fn) return cudaErrorNotSupported;
-  constexpr bool F16 = MODE != QGEMM_BF16, COMP = MODE == QGEMM_F16X3;
-  constexpr int BB = (QT == RG_TYPE_Q4_0) ? 18 : 34;
-  constexpr int NS = ring_depth(TN, COMP);
-  constexpr int NPL = COMP ? 2 : 1;
-  constexpr int RAW_ROW = 8 * BB;
-  alignas(64) CUtensorMap xmap, xlo_map, wmap;
+  alignas(64) CUtensorMap xmap, wmap;
   const cuuint32_t elem[2] = {1, 1};
-  for (int plane = 0; plane < NPL; ++plane) {
+  {
     const cuuint64_t dims[2] = {(cuuint64_t)a.k, (cuuint64_t)a.m};
     const cuuint64_t strides[1] = {(cuuint64_t)a.ldx * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)KSTEP, (cuuint32_t)(TN > 256 ? 256 : TN)};
-    if (fn(plane ? &xlo_map : &xmap, F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-           const_cast<void *>(plane ? a.x16_lo : a.x16), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint32_t box[2] = {(cuuint32_t)KSTEP, (cuuint32_t)(TN / 2)};
+    if (fn(&xmap, F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+           const_cast<void *>(a.x16), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return cudaErrorInvalidValue;
   }
-  if (!COMP) xlo_map = xmap;
   {
     const size_t row_bytes = (size_t)(a.k / 32) * BB;
     const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 8), (cuuint64_t)a.n};
@@ -413,10 +363,9 @@ cudaError_t launch_t(const QGemmArgs &a, const LaunchCfg &cfg) {
   P.split_stride = a.split_stride;
   P.status = cfg.status;
   P.accumulate = a.accumulate ? 1 : 0;
-  constexpr size_t smem =
-      1024 + NS * NPL * (A_BYTES + TN * KSTEP * 2) + RAW_NS * TM * RAW_ROW + (3 * NS + 2 * RAW_NS + 1) * 8 + 16;
+  constexpr size_t smem = 1024 + NS * (A_BYTES + B_BYTES) + RAW_NS * RAW_BYTES + (3 * NS + 2 * RAW_NS + 1) * 8 + 16;
   static_assert(smem <= 227 * 1024, "tile configuration exceeds the shared memory of one SM");
-  auto kernel = qgemm_tc_kernel<QT, TN, MODE>;
+  auto kernel = qgemm_tc_kernel<F16>;
   static DeviceOnce attr_once;  // per instantiation and device
   bool *attr_flag = attr_once.slot();
   if (!attr_flag || !*attr_flag) {
@@ -434,7 +383,7 @@ cudaError_t launch_t(const QGemmArgs &a, const LaunchCfg &cfg) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = at;
   lc.numAttrs = cfg.pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&lc, kernel, xmap, xlo_map, wmap, P);
+  return cudaLaunchKernelEx(&lc, kernel, xmap, wmap, P);
 }
 
 }  // namespace
@@ -449,7 +398,7 @@ bool qgemm_tc_wide_applies(const QGemmArgs &a) {
 cudaError_t launch_qgemm_tc_wide(const QGemmArgs &a, const LaunchCfg &cfg) {
   if (!qgemm_tc_wide_applies(a)) return cudaErrorInvalidValue;
   count_launch(LC_QGEMM_TC_WIDE);
-  return a.mode == QGEMM_BF16 ? launch_t<RG_TYPE_Q4_0, 512, QGEMM_BF16>(a, cfg) : launch_t<RG_TYPE_Q4_0, 512, QGEMM_F16>(a, cfg);
+  return a.mode == QGEMM_BF16 ? launch_t<false>(a, cfg) : launch_t<true>(a, cfg);
 }
 
 }  // namespace rg
