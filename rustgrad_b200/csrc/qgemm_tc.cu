@@ -108,11 +108,6 @@ __device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&v)
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -324,24 +319,23 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue
-    {
-      constexpr uint32_t idesc = umma_idesc(TM, TN, F16);
-      // One thread issues every MMA, so the loop is kept lean: a shared-memory descriptor is linear in the
-      // address (16-byte units), hence one base descriptor plus small constants per stage, K step and plane.
-      // The whole warp runs the loop and elects the issuing lane inside it: the operands of tcgen05.mma live in
-      // uniform registers, and under a branch on the lane every one of them is moved there anew for each MMA.
-      const uint64_t b_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(b_ring), 0));
-      const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-      for (int i = 0; i < nsteps; ++i) {
-        const int slot = i % NS;
-        const uint32_t ph = (uint32_t)((i / NS) & 1);
-        mbar_wait_bounded(&a_full[slot], ph, dead, P.status);
-        mbar_wait_bounded(&b_full[slot], ph, dead, P.status);
-        tc_fence_after();
-        const uint64_t b_desc = b_desc0 + (uint64_t)((slot * B_STAGE) >> 4);
-        const uint32_t a_tm = tmem_u + (uint32_t)(ACC_COLS + slot * A_STAGE_COLS);  // lane 0, first column of the stage
-        const uint32_t first = i > 0 ? 1u : 0u;  // the very first MMA of a tile overwrites the accumulator
-        if (elect_one()) {
+    constexpr uint32_t idesc = umma_idesc(TM, TN, F16);
+    // One thread issues every MMA, so the loop is kept lean: a shared-memory descriptor is linear in the
+    // address (16-byte units), hence one base descriptor plus small constants per stage, K step and plane.
+    // The whole warp runs the loop and elects the issuing lane inside it: the operands of tcgen05.mma live in
+    // uniform registers, and under a branch on the lane every one of them is moved there anew for each MMA.
+    const uint64_t b_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(b_ring), 0));
+    const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+    for (int i = 0; i < nsteps; ++i) {
+      const int slot = i % NS;
+      const uint32_t ph = (uint32_t)((i / NS) & 1);
+      mbar_wait_bounded(&a_full[slot], ph, dead, P.status);
+      mbar_wait_bounded(&b_full[slot], ph, dead, P.status);
+      tc_fence_after();
+      const uint64_t b_desc = b_desc0 + (uint64_t)((slot * B_STAGE) >> 4);
+      const uint32_t a_tm = tmem_u + (uint32_t)(ACC_COLS + slot * A_STAGE_COLS);  // lane 0, first column of the stage
+      const uint32_t first = i > 0 ? 1u : 0u;  // the very first MMA of a tile overwrites the accumulator
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < KSTEP / 16; ++kk) {
           const uint64_t b_hi = b_desc + (uint64_t)(kk * 2);  // 32 bytes per K step
@@ -359,11 +353,10 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
           }
         }
         umma_commit(&slot_free[slot]);  // the slot may be rewritten once these MMAs have read it
-        }
-        __syncwarp();
       }
-      if (elect_one()) umma_commit(acc_done);
+      __syncwarp();
     }
+    if (elect_one()) umma_commit(acc_done);
   } else {
     // ---------------------------------------------------------------- dequantisation: one block (half of a
     // stage's 64 columns) of one weight row per thread, two threads per row
@@ -381,46 +374,46 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
       uint32_t raw[RAW_ROW / 4];
 #pragma unroll
       for (int sub = 0; sub < RAW_STEPS; ++sub) {
-      const int i = i0 + sub, slot = i % NS;
-      const int v_lo = sub == 0 ? 0 : (sub * 2 * BB - 1) / 16 + 1, v_hi = ((sub + 1) * 2 * BB - 1) / 16;
+        const int i = i0 + sub, slot = i % NS;
+        const int v_lo = sub == 0 ? 0 : (sub * 2 * BB - 1) / 16 + 1, v_hi = ((sub + 1) * 2 * BB - 1) / 16;
 #pragma unroll
-      for (int v = v_lo; v <= v_hi; ++v) lds128(raw0 + (uint32_t)(rs * RT * RAW_BYTES + v * 16), &raw[4 * v]);
-      // pair layout: [d0 | q0] [d1 | q1] with a 2-byte scale in front of each block: the even block's
-      // quants straddle word boundaries (funnel shift), the odd block's are word aligned
-      const int w0 = sub * 2 * BB / 4;
-      uint32_t q[QW], dbits, vals[16];  // 32 values of this block, in k order
-      if (half == 0) {
+        for (int v = v_lo; v <= v_hi; ++v) lds128(raw0 + (uint32_t)(rs * RT * RAW_BYTES + v * 16), &raw[4 * v]);
+        // pair layout: [d0 | q0] [d1 | q1] with a 2-byte scale in front of each block: the even block's
+        // quants straddle word boundaries (funnel shift), the odd block's are word aligned
+        const int w0 = sub * 2 * BB / 4;
+        uint32_t q[QW], dbits, vals[16];  // 32 values of this block, in k order
+        if (half == 0) {
 #pragma unroll
-        for (int w = 0; w < QW; ++w) q[w] = __funnelshift_r(raw[w0 + w], raw[w0 + w + 1], 16);
-        dbits = raw[w0] & 0xffffu;
-      } else {
-        dbits = raw[w0 + QW] >> 16;
-#pragma unroll
-        for (int w = 0; w < QW; ++w) q[w] = raw[w0 + QW + 1 + w];
-      }
-      uint32_t lows[16];
-      if constexpr (COMP) {
-        if constexpr (Q4) {
-          q4_block_split(dbits, q, vals, lows);
+          for (int w = 0; w < QW; ++w) q[w] = __funnelshift_r(raw[w0 + w], raw[w0 + w + 1], 16);
+          dbits = raw[w0] & 0xffffu;
         } else {
-          q8_block_split(dbits, q, vals, lows);
+          dbits = raw[w0 + QW] >> 16;
+#pragma unroll
+          for (int w = 0; w < QW; ++w) q[w] = raw[w0 + QW + 1 + w];
         }
-      } else if constexpr (Q4) {
-        q4_block_to_16<F16>(dbits, q, vals);
-      } else {
-        q8_block_to_16<F16>(dbits, q, vals);
-      }
-      if (sub == RAW_STEPS - 1) mbar_arrive(&raw_free[rs]);  // the raw tile's last stage is in registers
-      if (i >= NS) mbar_wait_bounded(&slot_free[slot], (uint32_t)((i / NS - 1) & 1), dead, P.status);
-      tc_fence_after();
-      // this thread's block = 16 columns of its row's lane: [stage][plane][even block | odd block]
-      const uint32_t a_tm = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) +
-                            (uint32_t)(ACC_COLS + slot * A_STAGE_COLS + grp * A_TILE_COLS + half * 16);
-      tmem_store16(a_tm, vals);
-      if constexpr (COMP) tmem_store16(a_tm + A_COLS, lows);
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      tc_fence_before();
-      mbar_arrive(&a_full[slot]);
+        uint32_t lows[16];
+        if constexpr (COMP) {
+          if constexpr (Q4) {
+            q4_block_split(dbits, q, vals, lows);
+          } else {
+            q8_block_split(dbits, q, vals, lows);
+          }
+        } else if constexpr (Q4) {
+          q4_block_to_16<F16>(dbits, q, vals);
+        } else {
+          q8_block_to_16<F16>(dbits, q, vals);
+        }
+        if (sub == RAW_STEPS - 1) mbar_arrive(&raw_free[rs]);  // the raw tile's last stage is in registers
+        if (i >= NS) mbar_wait_bounded(&slot_free[slot], (uint32_t)((i / NS - 1) & 1), dead, P.status);
+        tc_fence_after();
+        // this thread's block = 16 columns of its row's lane: [stage][plane][even block | odd block]
+        const uint32_t a_tm = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) +
+                              (uint32_t)(ACC_COLS + slot * A_STAGE_COLS + grp * A_TILE_COLS + half * 16);
+        tmem_store16(a_tm, vals);
+        if constexpr (COMP) tmem_store16(a_tm + A_COLS, lows);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        mbar_arrive(&a_full[slot]);
       }
     }
     // ---------------------------------------------------------------- epilogue: TMEM -> global

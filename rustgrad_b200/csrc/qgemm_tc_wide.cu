@@ -74,11 +74,6 @@ __device__ __forceinline__ void umma_16bit(uint32_t tmem_d, uint64_t adesc, uint
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -207,22 +202,21 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue
-    {
-      // The whole warp runs the loop and elects the issuing lane inside it: the operands of tcgen05.mma live in uniform
-      // registers, and under a branch on the lane every one of them is moved there anew for each MMA.
-      const uint64_t a_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(a_ring), 0));
-      const uint64_t b_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(b_ring), 0));
-      const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-      // a 512-token tile is two 256-column accumulators fed by the same dequantised A tile
-      constexpr uint32_t idesc = umma_idesc(TM, TN / 2, F16);
-      for (int i = 0; i < nsteps; ++i) {
-        const int slot = i % NS;
-        const uint32_t ph = (uint32_t)((i / NS) & 1);
-        mbar_wait_bounded(&a_full[slot], ph, dead, P.status);
-        mbar_wait_bounded(&b_full[slot], ph, dead, P.status);
-        tc_fence_after();
-        const uint64_t a_desc = a_desc0 + (uint64_t)((slot * A_BYTES) >> 4), b_desc = b_desc0 + (uint64_t)((slot * B_BYTES) >> 4);
-        if (elect_one()) {
+    // The whole warp runs the loop and elects the issuing lane inside it: the operands of tcgen05.mma live in uniform
+    // registers, and under a branch on the lane every one of them is moved there anew for each MMA.
+    const uint64_t a_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(a_ring), 0));
+    const uint64_t b_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(b_ring), 0));
+    const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+    // a 512-token tile is two 256-column accumulators fed by the same dequantised A tile
+    constexpr uint32_t idesc = umma_idesc(TM, TN / 2, F16);
+    for (int i = 0; i < nsteps; ++i) {
+      const int slot = i % NS;
+      const uint32_t ph = (uint32_t)((i / NS) & 1);
+      mbar_wait_bounded(&a_full[slot], ph, dead, P.status);
+      mbar_wait_bounded(&b_full[slot], ph, dead, P.status);
+      tc_fence_after();
+      const uint64_t a_desc = a_desc0 + (uint64_t)((slot * A_BYTES) >> 4), b_desc = b_desc0 + (uint64_t)((slot * B_BYTES) >> 4);
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < KSTEP / 16; ++kk) {
           const uint64_t a_hi = a_desc + (uint64_t)(kk * 2), b_hi = b_desc + (uint64_t)(kk * 2);
@@ -230,11 +224,10 @@ __global__ void __launch_bounds__(THREADS, 1)
           umma_16bit(tmem_u + 256, a_hi, b_hi + (uint64_t)((256 * 128) >> 4), idesc, (i > 0 || kk > 0) ? 1u : 0u);
         }
         umma_commit(&slot_free[slot]);  // the slot may be rewritten once these MMAs have read it
-        }
-        __syncwarp();
       }
-      if (elect_one()) umma_commit(acc_done);
+      __syncwarp();
     }
+    if (elect_one()) umma_commit(acc_done);
   } else {
     // ---------------------------------------------------------------- dequantisation: one block (half of a
     // stage's 64 columns) of one weight row per thread, two threads per row
