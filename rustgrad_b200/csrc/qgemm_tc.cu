@@ -664,6 +664,7 @@ cudaError_t launch_to16(const float *x, int ldx, int k, int rows, const Operand1
 
 cudaError_t launch_reduce_splits(const float *part, int splits, size_t stride, int n, int rows, float *out, int ldo, bool accumulate,
                                  const LaunchCfg &cfg) {
+  count_launch(LC_REDUCE_SPLITS);
   return launch_simple(accumulate ? reduce_splits_kernel<true> : reduce_splits_kernel<false>,
                        dim3((unsigned)((n + 255) / 256), (unsigned)rows), dim3(256), cfg, part, splits, stride, n, out, ldo);
 }

@@ -694,8 +694,8 @@ def test_batched_prompt_prefill_matches_per_prompt_prefill(small_hd128, tiny):
     """Several prompts in one pass (rg_b200_prefill_rows; src/models/transformer/batch.rs:177-325):
     one chunk holding five prompts of very different lengths (logits of five arbitrary columns),
     prompts cut across two chunks, a row that continues from cached positions, and a model that is
-    not on the tensor-core path; every prompt must see exactly what it sees alone, and the decode
-    step that follows must find every cache row in place."""
+    not on the tensor-core path; every prompt must give the logits of the checker's run of it alone, within
+    the bar, and the decode step that follows must find every cache row in place."""
     cfg, tensors = small_hd128
     mk = lambda **kw: session.LlamaCudaPlan.from_tensors(  # noqa: E731
         cfg, tensors, session.CudaSessionTarget(kv_f32=True, max_context=1100, **kw)).prepare()
@@ -813,19 +813,47 @@ def test_batched_decode_attention_on_tensor_cores_with_f16_cache(heads, kv_heads
         assert session.launch_count("attn_decode_tc") >= before + cfg["n_layers"]  # later steps may replay a captured graph
 
 
-@pytest.mark.parametrize("n", [9, 32, 33, 64, 65, 128, 129, 257])
+@pytest.mark.parametrize("n", [9, 16, 17, 32, 33, 64, 65, 128, 129, 257])
 @pytest.mark.parametrize("body", [quant.Q4_0, quant.Q8_0], ids=["q4_0", "q8_0"])
-def test_prompts_around_the_token_tiles_with_the_projections_split_over_k(n, body):
-    """Prompts whose projections have fewer output tiles than the GPU has SMs: K is split over CTAs and the partial
-    sums are added in split order, into the residual stream where the projection ends there.  Token counts at the
-    edges of the 16 / 32 / 64 / 128-column tiles; stacked and unstacked weights go through the same rule."""
+def test_prompts_around_the_token_tiles(n, body):
+    """Token counts at the edges of the 16 / 32 / 64 / 128-column tiles.  Up to 32 tokens all seven projections of a
+    layer split K over CTAs (one 256-column piece each here) and a second launch adds the partial sums in split order,
+    into the residual stream where the projection ends there; above that none does."""
     cfg = synth.scaled(synth.TINY, d_model=1024, n_heads=8, n_kv_heads=2, head_dim=128, ffn_dim=2304, vocab=640, n_layers=2,
                        rope_theta=500000.0, max_context=272)
     tensors = synth.build_tensors(cfg, seed=9, body_type=body, embed_type=quant.Q8_0, head_type=quant.Q8_0, tied_head=False)
     prompt = synth.prompt_ids(cfg, n, seed=n)
     want = O.OracleModel(cfg, tensors, threads=4).forward(prompt, O.MODE_FAST)
     s = session.LlamaCudaPlan.from_tensors(cfg, tensors, session.CudaSessionTarget(kv_f32=True, max_context=272)).prepare()
+    before = session.launch_count("reduce_splits")
     assert_logits_close(s.prefill_ids(prompt), want)
+    assert session.launch_count("reduce_splits") == before + (7 * cfg["n_layers"] if n <= 32 else 0)
+
+
+@pytest.fixture(scope="module", params=[quant.Q4_0, quant.Q8_0], ids=["q4_0", "q8_0"])
+def wide_layer(request):
+    """One layer whose matrices are tall enough for K parts of several 256-column pieces (148 SMs): gate and up 4 parts
+    of 2, down 20 of 2 with a last one of 1 (added into the residual stream), the vocabulary head 3 parts of 3, 3
+    and 2, which go around the two-piece ring of raw weight tiles."""
+    cfg = synth.scaled(synth.TINY, d_model=2048, n_heads=16, n_kv_heads=4, head_dim=128, ffn_dim=9984, vocab=20000, n_layers=1,
+                       rope_theta=500000.0, max_context=64)
+    return cfg, synth.build_tensors(cfg, seed=12, body_type=request.param, embed_type=quant.Q8_0, head_type=request.param, tied_head=False)
+
+
+@pytest.mark.parametrize("lengths", [(20,), (9, 8, 15), (1,) * 32, (1,) * 8 + (2,) * 9, (30, 10, 3)], ids=lambda v: f"{len(v)}x{sum(v)}")
+def test_uneven_k_parts_of_short_prompts(wide_layer, lengths):
+    """Products of up to 32 columns cut K into parts of unequal length: the prompts of one chunk against the checker,
+    and the number of reductions: one per projection of a chunk of up to 32 columns, one for a head of 3 to 32 rows."""
+    cfg, tensors = wide_layer
+    s = session.LlamaCudaPlan.from_tensors(cfg, tensors, session.CudaSessionTarget(kv_f32=True, max_batch=32, max_context=64)).prepare()
+    prompts = {r: synth.prompt_ids(cfg, n, seed=50 + r) for r, n in enumerate(lengths)}
+    before = session.launch_count("reduce_splits")
+    logits, greedy = s.prefill_rows(prompts)
+    assert session.launch_count("reduce_splits") == before + (7 if sum(lengths) <= 32 else 0) + (1 if len(lengths) >= 3 else 0)
+    for r, p in prompts.items():
+        want = O.OracleModel(cfg, tensors, threads=4).forward(p, O.MODE_FAST)
+        assert_logits_close(logits[r], want)
+        assert int(greedy[r]) == O.select_greedy(want)
 
 
 @pytest.mark.parametrize("kv_f32", [False, True], ids=["kv_f16", "kv_f32"])
