@@ -857,16 +857,16 @@ def test_uneven_k_parts_of_short_prompts(wide_layer, lengths):
 
 
 @pytest.mark.parametrize("kv_f32", [False, True], ids=["kv_f16", "kv_f32"])
-@pytest.mark.parametrize("n", [33, 64, 65, 117, 200])
-def test_a_prompt_leaves_the_same_cache_rows_whatever_shares_its_chunk(n, kv_f32):
-    """Prompt chunks of more than 32 columns add every token's products up in one fixed order, so what a prompt leaves
-    in its cache row does not depend on the prompts it is prefilled with.  The logits of the decode step behind it see
+@pytest.mark.parametrize("n,others", [(9, 7), (9, 23), (17, 15), (33, 500), (64, 500), (65, 500), (117, 500), (200, 500)])
+def test_a_prompt_leaves_the_same_cache_rows_whatever_shares_its_chunk(n, others, kv_f32):
+    """Prompt chunks of 9 to 32 columns, and those of more, add every token's products up in one fixed order each, so what a
+    prompt leaves in its cache row does not depend on the prompts it is prefilled with.  The logits of the decode step behind it see
     the caches alone: they are the same bits for the prompt by itself, in front of another one and behind it.  The
     model's projections have from 8 to 78 row tiles for that many tokens, far fewer than the GPU has SMs."""
     cfg = synth.scaled(synth.TINY, d_model=2048, n_heads=16, n_kv_heads=4, head_dim=128, ffn_dim=9984, vocab=640, n_layers=2,
                        rope_theta=500000.0, max_context=600)
     s = session.LlamaCudaPlan.synthetic(cfg, session.CudaSessionTarget(kv_f32=kv_f32, max_batch=2, max_context=600), seed=5).prepare()
-    prompt, other = synth.prompt_ids(cfg, n, seed=n), synth.prompt_ids(cfg, 500, seed=1)
+    prompt, other = synth.prompt_ids(cfg, n, seed=n), synth.prompt_ids(cfg, others, seed=1)
     behind = []
     for fill in (lambda: s.prefill_ids(prompt, row=0, want_logits=False), lambda: s.prefill_rows({0: prompt, 1: other}, want_logits=False),
                  lambda: s.prefill_rows({1: other, 0: prompt}, want_logits=False)):
