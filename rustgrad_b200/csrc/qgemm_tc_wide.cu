@@ -3,9 +3,9 @@
 // One CTA computes 128 weight rows x 512 tokens: the dequantised A tile (K-major, 128-byte swizzle, in
 // SHARED memory) feeds two 256-column accumulators that together fill tensor memory, so each weight
 // block is expanded once per 512 tokens.  With all 512 TMEM columns taken by the accumulators the A
-// operand cannot live in tensor memory as it does in qgemm_tc.cu; measured on [14336,4096] x 2048 bf16
-// this tile shape still wins (267 us against 286 us), and on [4096,4096] x 2048 it runs a single wave
-// (66 us against 87 us).  Warp roles, rings and bounded waits are those of qgemm_tc.cu.
+// operand cannot live in tensor memory as it does in qgemm_tc.cu.  Warp roles, rings and bounded waits are those of
+// qgemm_tc.cu.  bf16 against its 128 x 256 tiles: one wave of wide tiles is faster ([14336,4096] x 512 68 us against 70,
+// x 257 59 against 63; [4096,4096] x 2048 66 against 70), several waves are not ([14336,4096] x 2048 264 against 230).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -383,7 +383,8 @@ cudaError_t launch_t(const QGemmArgs &a, const LaunchCfg &cfg) {
 
 bool qgemm_tc_wide_applies(const QGemmArgs &a) {
   if (!(a.type == RG_TYPE_Q4_0 && a.mode != QGEMM_F16X3 && a.m > 256 && a.splits <= 1)) return false;
-  // with few CTAs the 256-token tiles of qgemm_tc.cu fill more SMs
+  // with few CTAs the 256-token tiles of qgemm_tc.cu fill more SMs ([4096,4096] x 512: 35 us on 64 of them).  The bound was
+  // set when that kernel was slower in several waves too (286 us against 267 on [14336,4096] x 2048, now 230 against 264).
   const long ctas = (long)((a.n + TM - 1) / TM) * (long)((a.m + 511) / 512);
   return ctas >= 96;
 }
