@@ -8,19 +8,23 @@
 //   * MMA M = 128 weight rows (the dequantised tile is the A operand), MMA N = TN tokens (the
 //     activation tile is the B operand), K = 16 per tcgen05.mma, four per 64-element stage;
 //     the accumulator lives in TMEM (128 lanes x TN f32 columns).
-//   * warp 0: TMA producer.  Activation tiles come as tiled 2-D copies with the 128-byte swizzle;
-//     the raw block bytes of the 128 weight rows, 256 columns (8 blocks) at a time, come through
-//     a second tiled 2-D map into a small ring, so no thread waits on global memory.
-//   * warp 1: allocates TMEM, issues tcgen05.mma from one thread, commits to mbarriers.
-//   * warps 2-17 (two groups of eight taking alternate stages): two threads per weight row; each expands one block per stage (nibbles to exact
+//   * warp 0: TMA producer of the activation tiles (tiled 2-D copies with the 128-byte swizzle); the last warp: TMA
+//     producer of the raw block bytes of the 128 weight rows, 256 columns (8 blocks) at a time, through a second tiled
+//     2-D map into a small ring, so no thread waits on global memory.
+//   * warp 1: allocates TMEM, issues tcgen05.mma from one lane, commits to mbarriers.
+//   * eight warps a row tile: two threads per weight row, one for the even and one for the odd block of a stage; each expands one
+//     block per stage (nibbles to exact
 //     16-bit integers by bit pattern, one packed subtract and one packed multiply by the block
 //     scale per two weights) and writes its 32 values with tcgen05.st straight into TENSOR MEMORY:
 //     the A operand of the MMA is read from TMEM (lane = weight row, one 32-bit column per two K
 //     values), so the dequantised weights never pass through shared memory, whose bandwidth is
 //     then left to the activation tiles.  Afterwards the same warps read the accumulator with
 //     tcgen05.ld and store it.
-//   * Operand rings of 3-4 stages with bounded mbarrier waits; a time-out records a status and
+//   * Operand rings of 2-4 stages with bounded mbarrier waits; a time-out records a status and
 //     the kernel still frees its TMEM and exits.
+// What bounds it: the tensor cores for tiles of 128 tokens (1 536 of 1 750 cycles a step with two row tiles), the issue loop of the
+// MMA warp and the dequantisation for narrow ones (about 700 cycles a step for 222 of MMAs at 32 tokens, two CTAs an SM).
+// Measured for M = 128 with A in tensor memory: 14 / 18 / 32 / 64 cycles an MMA for N = 16 / 32 / 64 / 128.
 // Operand modes: bf16 (weights enter as bf16(bf16(d) * (n - 8)) for Q4_0), f16 (weights enter as
 // f16(d * (n - 8))), and compensated f16, where every operand is the sum of two halves
 // (hi = f16(v), lo = f16(v - hi)) and each K step issues hi.hi + hi.lo + lo.hi into the same
@@ -41,13 +45,6 @@ namespace {
 constexpr int TM = 128;       // weight rows per tile (MMA M)
 constexpr int KSTEP = 64;     // elements per stage (128 bytes: one swizzle row)
 constexpr int RAW_STEPS = 4;  // 64-element stages per raw weight tile (256 columns = 8 blocks)
-constexpr int RAW_NS = 2;     // raw ring depth
-// RT = row tiles of 128 weight rows per CTA.  The compensated mode moves two activation planes per stage and is
-// bound by that traffic from L2, so there one activation tile feeds two row tiles (RT = 2, at most 128 tokens);
-// the single-operand modes are bound by the dequantisation and prefer one row tile against 256 tokens.
-constexpr int MAX_THREADS = 64 + 2 * 256;  // TMA warp, MMA warp, eight dequantisation / epilogue warps per row tile
-constexpr int A_COLS = KSTEP / 2;  // TMEM columns of one dequantised A stage (two 16-bit values per column)
-
 struct Params {
   int n, k;     // weight rows, columns
   int m;        // tokens
@@ -105,12 +102,34 @@ __device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&v)
       "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
 }
+// Two planes of a block (hi, lo), 16 columns each, side by side.
+__device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&v)[16], const uint32_t (&w)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+      "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]), "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+      : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// mbar_wait_bounded for a whole warp whose lanes wait on barriers of their own.
+__device__ __forceinline__ bool wait_lanes(uint64_t *bar, uint32_t parity, volatile int *dead, int *status, uint32_t limit = (1u << 22)) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  for (uint32_t i = 0; i < limit; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 1023u) == 0u && __any_sync(0xffffffffu, *dead)) return false;
+  }
+  *dead = 1;
+  if (status) atomicExch(status, DEV_TIMEOUT);
+  return false;
+}
 
 __device__ __forceinline__ void lds128(uint32_t addr, uint32_t *v) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
@@ -193,20 +212,21 @@ __device__ __forceinline__ void q8_block_to_16(uint32_t dbits16, const uint32_t 
 // fused multiply-add (Q4_0: q * d - hi is exact before its single rounding).
 __device__ __forceinline__ void q4_block_split(uint32_t dbits16, const uint32_t (&q)[4], uint32_t (&hi)[16], uint32_t (&lo)[16]) {
   const uint32_t d2 = dbits16 | (dbits16 << 16);
-  const uint32_t M = 0x000F000Fu, E = 0x64006400u, OFF = 0x64086408u;
+  const uint32_t E = 0x64006400u;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint32_t w = prmt(q[i], 0u, 0x3120u);
-    const uint32_t n[4] = {w & M, (w >> 8) & M, (w >> 4) & M, (w >> 12) & M};
+    const uint32_t w = prmt(q[i], 0u, 0x3120u), ws = w >> 8;
+    // low nibbles: (1024 | n) - 1032; high nibbles stay in place: (1024 | 16 n) / 16 - 72.  Both give n - 8 exactly.
+    const uint32_t qf[4] = {hsub2_u32((w & 0x000F000Fu) | E, 0x64086408u), hsub2_u32((ws & 0x000F000Fu) | E, 0x64086408u),
+                            hfma2_u32((w & 0x00F000F0u) | E, 0x2C002C00u, 0xD480D480u),
+                            hfma2_u32((ws & 0x00F000F0u) | E, 0x2C002C00u, 0xD480D480u)};
     const int slot[4] = {2 * i, 2 * i + 1, 8 + 2 * i, 8 + 2 * i + 1};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const uint32_t qf = sub2<true>(n[j] | E, OFF);
-      const uint32_t h = mul2<true>(qf, d2);
-      uint32_t l;
-      asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(l) : "r"(qf), "r"(d2), "r"(h ^ 0x80008000u));
-      hi[slot[j]] = h;
-      lo[slot[j]] = l;
+      const __half2 f = *reinterpret_cast<const __half2 *>(&qf[j]), d = *reinterpret_cast<const __half2 *>(&d2);
+      const __half2 h = __hmul2(f, d), l = __hfma2(f, d, __hneg2(h));  // the negation rides in the instruction
+      hi[slot[j]] = *reinterpret_cast<const uint32_t *>(&h);
+      lo[slot[j]] = *reinterpret_cast<const uint32_t *>(&l);
     }
   }
 }
@@ -231,39 +251,63 @@ __device__ __forceinline__ void q8_block_split(uint32_t dbits16, const uint32_t 
   }
 }
 
-// Ring depth of the activation tiles (shared memory) and of the dequantised A stages (tensor memory).
-__host__ __device__ constexpr int ring_depth(int tn, bool comp) { return comp ? (tn >= 64 ? 2 : 3) : 4; }  // tensor-memory budget
-__host__ __device__ constexpr int row_tiles(int mode) { return mode == QGEMM_F16X3 ? 2 : 1; }
-__host__ __device__ constexpr int pow2_cols(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512; }
+__host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
+
+// What one CTA holds.  The A operand travels through tensor memory in stages of two 32-element blocks (16 columns a plane
+// each), which the two halves of a row tile's dequantisation warps fill on their own; a step's MMAs release its stage of A and of
+// the activations with one commit (three commits and three waits a step were half of the MMA warp's loop).
+// The activation ring (64 elements a stage) and the raw weight ring have barriers and a producing warp of their own: with
+// one warp for both, the raw tile of steps 4j.. was asked for only when the MMAs of step 4j - 3 were done.
+template <int QT, int TN, int MODE, int RT>
+struct Tile {
+  static constexpr bool Q4 = (QT == RG_TYPE_Q4_0);
+  static constexpr bool F16 = MODE != QGEMM_BF16, COMP = MODE == QGEMM_F16X3;
+  static constexpr int NPL = COMP ? 2 : 1;  // operand planes per stage: hi (and lo)
+  static constexpr int BB = Q4 ? 18 : 34;
+  static constexpr int B_BYTES = TN * KSTEP * 2;
+  static constexpr int B_STAGE = NPL * B_BYTES;
+  static constexpr int RAW_ROW = 8 * BB;  // bytes of one weight row in a raw tile (144 / 272)
+  static constexpr int RAW_BYTES = TM * RAW_ROW;
+  static constexpr int A_BLK = NPL * 16;  // tensor-memory columns of one row tile's block (hi, lo)
+  static constexpr int A_SLOT = RT * A_BLK;
+  static constexpr int ACC_T = TN < 32 ? 32 : TN;  // accumulator columns of one row tile
+  static constexpr int ACC_COLS = RT * ACC_T;      // accumulators first, then the A ring
+  static constexpr int EXTRA = 1024 + 512;         // alignment of the rings, barriers
+  // Two CTAs share an SM where two stages of both rings fit half of its shared memory: one dequantises while the other's
+  // waits run out.
+  static constexpr bool PAIR = RT == 1 && TN <= 128 && EXTRA + 2 * B_STAGE + 2 * RT * RAW_BYTES <= 113 * 1024;
+  static constexpr int SMEM = PAIR ? 113 * 1024 : 227 * 1024;
+  static constexpr int TMEM_COLS = PAIR ? 256 : 512;
+  static constexpr int NSA = cmin(4, (TMEM_COLS - ACC_COLS) / (2 * A_SLOT));  // stages of two blocks
+  static constexpr int NSB = cmin(4, (SMEM - EXTRA - 2 * RT * RAW_BYTES) / B_STAGE);
+  static constexpr int RAW_NS = cmin(3, (SMEM - EXTRA - NSB * B_STAGE) / (RT * RAW_BYTES));
+  static constexpr int ND = NSA > NSB ? NSA : NSB;  // barriers that say a step's MMAs are over
+  static constexpr int SMEM_BYTES = EXTRA + NSB * B_STAGE + RAW_NS * RT * RAW_BYTES;
+  static constexpr int DQ_WARPS = 8 * RT;
+  static constexpr int THREADS = (DQ_WARPS + 3) * 32;  // activation TMA, MMA, dequantisation / epilogue, raw weight TMA
+  static_assert(ACC_COLS + NSA * 2 * A_SLOT <= TMEM_COLS && NSA >= 2, "tensor memory budget");
+  static_assert(NSB >= 2 && RAW_NS >= 2 && SMEM_BYTES <= SMEM, "shared memory budget");
+};
 
 template <int QT, int TN, int MODE, int RT>
-__global__ void __launch_bounds__(MAX_THREADS, 1)
+__global__ void __launch_bounds__((Tile<QT, TN, MODE, RT>::THREADS), (Tile<QT, TN, MODE, RT>::PAIR ? 2 : 1))
     qgemm_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap xlo_map,
                     const __grid_constant__ CUtensorMap wmap, const Params P) {
-  constexpr bool Q4 = (QT == RG_TYPE_Q4_0);
-  constexpr bool F16 = MODE != QGEMM_BF16, COMP = MODE == QGEMM_F16X3;
-  constexpr int NPL = COMP ? 2 : 1;  // operand planes per stage: hi (and lo)
-  constexpr int BB = Q4 ? 18 : 34;
-  constexpr int NS = ring_depth(TN, COMP);  // operand ring depth
-  constexpr int B_BYTES = TN * KSTEP * 2;
-  constexpr int B_STAGE = NPL * B_BYTES;
-  constexpr int A_TILE_COLS = NPL * A_COLS;       // TMEM columns of one row tile's A stage (hi, lo)
-  constexpr int A_STAGE_COLS = RT * A_TILE_COLS;  // both row tiles
-  constexpr int RAW_ROW = 8 * BB;  // bytes of one weight row in a raw tile (144 / 272)
-  constexpr int RAW_BYTES = TM * RAW_ROW;
-  constexpr int ACC_T = TN < 32 ? 32 : TN;  // accumulator columns of one row tile
-  constexpr int ACC_COLS = RT * ACC_T;      // accumulators first, then the A ring
-  constexpr int TMEM_COLS = pow2_cols(ACC_COLS + NS * A_STAGE_COLS);
-  static_assert(ACC_COLS + NS * A_STAGE_COLS <= 512, "tensor memory budget");
+  using T = Tile<QT, TN, MODE, RT>;
+  constexpr bool Q4 = T::Q4, F16 = T::F16, COMP = T::COMP;
+  constexpr int BB = T::BB, NSA = T::NSA, NSB = T::NSB, ND = T::ND, RAW_NS = T::RAW_NS;
+  constexpr int B_BYTES = T::B_BYTES, B_STAGE = T::B_STAGE, RAW_ROW = T::RAW_ROW, RAW_BYTES = T::RAW_BYTES;
+  constexpr int ACC_T = T::ACC_T, ACC_COLS = T::ACC_COLS, A_BLK = T::A_BLK, A_SLOT = T::A_SLOT;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t *b_ring = smem;
-  uint8_t *raw_ring = b_ring + NS * B_STAGE;
+  uint8_t *raw_ring = b_ring + NSB * B_STAGE;
   uint64_t *bars = reinterpret_cast<uint64_t *>(raw_ring + RAW_NS * RT * RAW_BYTES);
-  uint64_t *b_full = bars, *a_full = bars + NS, *slot_free = bars + 2 * NS;
-  uint64_t *raw_full = bars + 3 * NS, *raw_free = raw_full + RAW_NS, *acc_done = raw_free + RAW_NS;
+  uint64_t *b_full = bars, *a_full = b_full + NSB /* [stage][block] */, *done = a_full + 2 * NSA;
+  uint64_t *raw_full = done + ND, *raw_free = raw_full + RAW_NS, *acc_done = raw_free + RAW_NS;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_done + 1);
   volatile int *dead = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  static_assert((NSB + 2 * NSA + ND + 2 * RAW_NS + 1) * 8 + 8 <= 512, "barriers");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * (TM * RT), tok0 = blockIdx.y * TN;
@@ -271,21 +315,19 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
   const int nsteps = min(P.k_steps, P.k / KSTEP - step0);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NS; ++s) {
-      mbar_init(&b_full[s], 1);
-      mbar_init(&a_full[s], RT * 256);
-      mbar_init(&slot_free[s], 1);
-    }
+    for (int s = 0; s < NSB; ++s) mbar_init(&b_full[s], 1);
+    for (int s = 0; s < 2 * NSA; ++s) mbar_init(&a_full[s], RT * 4);  // the four warps of a block in every row tile
+    for (int s = 0; s < ND; ++s) mbar_init(&done[s], 1);
     for (int s = 0; s < RAW_NS; ++s) {
       mbar_init(&raw_full[s], 1);
-      mbar_init(&raw_free[s], RT * 256);
+      mbar_init(&raw_free[s], T::DQ_WARPS);
     }
     mbar_init(acc_done, 1);
     *dead = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(TMEM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(T::TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -294,27 +336,39 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
-  pdl_wait();
 
   if (warp == 0) {
-    // ---------------------------------------------------------------- TMA: raw weight tiles and activation tiles
+    // ---------------------------------------------------------------- TMA: activation tiles (an earlier kernel's output)
     if (lane == 0) {
+      pdl_wait();
+      int slot = 0, d = 0;
+      uint32_t pd = 0;
       for (int i = 0; i < nsteps; ++i) {
-        if (i % RAW_STEPS == 0) {
-          const int j = i / RAW_STEPS, rs = j % RAW_NS;
-          if (j >= RAW_NS) mbar_wait_bounded(&raw_free[rs], (uint32_t)((j / RAW_NS - 1) & 1), dead, P.status);
-          mbar_expect_tx(&raw_full[rs], (uint32_t)(RT * RAW_BYTES));
-          // x in 8-byte elements; rows beyond the tensor arrive as zeros (zero scale, zero weights)
-#pragma unroll
-          for (int t = 0; t < RT; ++t)
-            tma_tile_2d(raw_ring + (rs * RT + t) * RAW_BYTES, &wmap, ((step0 + i) / RAW_STEPS) * (RAW_ROW / 8), n0 + t * TM,
-                        &raw_full[rs]);
+        if (i >= NSB) {  // step i - NSB has read the slot
+          mbar_wait_bounded(&done[d], pd, dead, P.status);
+          if (++d == ND) {
+            d = 0;
+            pd ^= 1u;
+          }
         }
-        const int slot = i % NS;
-        if (i >= NS) mbar_wait_bounded(&slot_free[slot], (uint32_t)((i / NS - 1) & 1), dead, P.status);
         mbar_expect_tx(&b_full[slot], (uint32_t)B_STAGE);
         tma_tile_2d(b_ring + slot * B_STAGE, &xmap, (step0 + i) * KSTEP, tok0, &b_full[slot]);
         if constexpr (COMP) tma_tile_2d(b_ring + slot * B_STAGE + B_BYTES, &xlo_map, (step0 + i) * KSTEP, tok0, &b_full[slot]);
+        if (++slot == NSB) slot = 0;
+      }
+    }
+  } else if (warp == T::DQ_WARPS + 2) {
+    // ---------------------------------------------------------------- TMA: raw weight tiles (constant: no wait for earlier kernels)
+    if (lane == 0) {
+      for (int j = 0; j * RAW_STEPS < nsteps; ++j) {
+        const int rs = j % RAW_NS;
+        if (j >= RAW_NS) mbar_wait_bounded(&raw_free[rs], (uint32_t)((j / RAW_NS - 1) & 1), dead, P.status);
+        mbar_expect_tx(&raw_full[rs], (uint32_t)(RT * RAW_BYTES));
+        // x in 8-byte elements; rows beyond the tensor arrive as zeros (zero scale, zero weights)
+#pragma unroll
+        for (int t = 0; t < RT; ++t)
+          tma_tile_2d(raw_ring + (rs * RT + t) * RAW_BYTES, &wmap, (step0 / RAW_STEPS + j) * (RAW_ROW / 8), n0 + t * TM,
+                      &raw_full[rs]);
       }
     }
   } else if (warp == 1) {
@@ -326,14 +380,15 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
     // uniform registers, and under a branch on the lane every one of them is moved there anew for each MMA.
     const uint64_t b_desc0 = umma_desc(__shfl_sync(0xffffffffu, smem_u32(b_ring), 0));
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int sa = 0, sb = 0, d = 0;
+    uint32_t pa = 0, pb = 0;
     for (int i = 0; i < nsteps; ++i) {
-      const int slot = i % NS;
-      const uint32_t ph = (uint32_t)((i / NS) & 1);
-      mbar_wait_bounded(&a_full[slot], ph, dead, P.status);
-      mbar_wait_bounded(&b_full[slot], ph, dead, P.status);
+      // Three barriers, one poll: lanes 0 and 1 ask for the two blocks of A, the others for B.  One after the other they took
+      // longer than the MMAs of a narrow tile.
+      wait_lanes(lane < 2 ? &a_full[2 * sa + lane] : &b_full[sb], lane < 2 ? pa : pb, dead, P.status);
       tc_fence_after();
-      const uint64_t b_desc = b_desc0 + (uint64_t)((slot * B_STAGE) >> 4);
-      const uint32_t a_tm = tmem_u + (uint32_t)(ACC_COLS + slot * A_STAGE_COLS);  // lane 0, first column of the stage
+      const uint64_t b_desc = b_desc0 + (uint64_t)((sb * B_STAGE) >> 4);
+      const uint32_t a_tm = tmem_u + (uint32_t)(ACC_COLS + sa * 2 * A_SLOT);  // lane 0, first column of the stage
       const uint32_t first = i > 0 ? 1u : 0u;  // the very first MMA of a tile overwrites the accumulator
       if (elect_one()) {
 #pragma unroll
@@ -342,19 +397,28 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
 #pragma unroll
           for (int t = 0; t < RT; ++t) {
             const uint32_t acc = tmem_u + t * ACC_T;
-            const uint32_t a_hi = a_tm + t * A_TILE_COLS + kk * 8;  // 16 K values = 8 columns
+            const uint32_t a_hi = a_tm + (kk / 2) * A_SLOT + t * A_BLK + (kk & 1) * 8;  // 16 K values = 8 columns
             if constexpr (COMP) {  // the small terms first, then hi.hi
               umma_16bit_ta(acc, a_hi, b_hi + (uint64_t)(B_BYTES >> 4), idesc, kk > 0 ? 1u : first);
-              umma_16bit_ta(acc, a_hi + A_COLS, b_hi, idesc, 1u);
+              umma_16bit_ta(acc, a_hi + 16, b_hi, idesc, 1u);
               umma_16bit_ta(acc, a_hi, b_hi, idesc, 1u);
             } else {
               umma_16bit_ta(acc, a_hi, b_hi, idesc, kk > 0 ? 1u : first);
             }
           }
         }
-        umma_commit(&slot_free[slot]);  // the slot may be rewritten once these MMAs have read it
+        umma_commit(&done[d]);  // the step's slots of both rings may be rewritten once these MMAs have read them
       }
       __syncwarp();
+      if (++sa == NSA) {
+        sa = 0;
+        pa ^= 1u;
+      }
+      if (++sb == NSB) {
+        sb = 0;
+        pb ^= 1u;
+      }
+      if (++d == ND) d = 0;
     }
     if (elect_one()) umma_commit(acc_done);
   } else {
@@ -366,15 +430,16 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
     const int grp = (warp - 2) >> 3;         // row tile of this warp
     constexpr int QW = Q4 ? 4 : 8;             // quant words per block
     const uint32_t raw0 = smem_u32(raw_ring) + (uint32_t)(grp * RAW_BYTES + r * RAW_ROW);
+    const uint32_t a_tm0 = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(ACC_COLS + grp * A_BLK);
+    int sa = 0, rs = 0, d = 0;
+    uint32_t pd = 0, praw = 0;
     for (int i0 = 0; i0 < nsteps; i0 += RAW_STEPS) {  // nsteps is a multiple of RAW_STEPS
-      const int j = i0 / RAW_STEPS, rs = j % RAW_NS;
-      mbar_wait_bounded(&raw_full[rs], (uint32_t)((j / RAW_NS) & 1), dead, P.status);
+      mbar_wait_bounded(&raw_full[rs], praw, dead, P.status);
       // The row is read 16 bytes at a time, each once per thread: a row pitch of 144 / 272 bytes spreads such reads over
       // all banks, where 4-byte reads met four to a bank.
       uint32_t raw[RAW_ROW / 4];
 #pragma unroll
       for (int sub = 0; sub < RAW_STEPS; ++sub) {
-        const int i = i0 + sub, slot = i % NS;
         const int v_lo = sub == 0 ? 0 : (sub * 2 * BB - 1) / 16 + 1, v_hi = ((sub + 1) * 2 * BB - 1) / 16;
 #pragma unroll
         for (int v = v_lo; v <= v_hi; ++v) lds128(raw0 + (uint32_t)(rs * RT * RAW_BYTES + v * 16), &raw[4 * v]);
@@ -403,22 +468,40 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
         } else {
           q8_block_to_16<F16>(dbits, q, vals);
         }
-        if (sub == RAW_STEPS - 1) mbar_arrive(&raw_free[rs]);  // the raw tile's last stage is in registers
-        if (i >= NS) mbar_wait_bounded(&slot_free[slot], (uint32_t)((i / NS - 1) & 1), dead, P.status);
+        if (sub == RAW_STEPS - 1) {  // the raw tile's last stage is in registers
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&raw_free[rs]);
+        }
+        if (i0 + sub >= NSA) {  // step i0 + sub - NSA has read the stage
+          mbar_wait_bounded(&done[d], pd, dead, P.status);
+          if (++d == ND) {
+            d = 0;
+            pd ^= 1u;
+          }
+        }
         tc_fence_after();
-        // this thread's block = 16 columns of its row's lane: [stage][plane][even block | odd block]
-        const uint32_t a_tm = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) +
-                              (uint32_t)(ACC_COLS + slot * A_STAGE_COLS + grp * A_TILE_COLS + half * 16);
-        tmem_store16(a_tm, vals);
-        if constexpr (COMP) tmem_store16(a_tm + A_COLS, lows);
+        // this thread's block of its row's lane: 16 columns a plane
+        const uint32_t a_tm = a_tm0 + (uint32_t)((2 * sa + half) * A_SLOT);
+        if constexpr (COMP) {
+          tmem_store32(a_tm, vals, lows);
+        } else {
+          tmem_store16(a_tm, vals);
+        }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
-        mbar_arrive(&a_full[slot]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_full[2 * sa + half]);
+        if (++sa == NSA) sa = 0;
+      }
+      if (++rs == RAW_NS) {
+        rs = 0;
+        praw ^= 1u;
       }
     }
     // ---------------------------------------------------------------- epilogue: TMEM -> global
     mbar_wait_bounded(acc_done, 0, dead, P.status);
     tc_fence_after();
+    pdl_wait();
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31 belong to this warp
     const int orow = n0 + grp * TM + quarter * 32 + lane;  // this warp's row tile
     float *out = P.out + (size_t)blockIdx.z * P.split_stride;
@@ -433,14 +516,20 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
               "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
             : "r"(taddr));
+        float *dst = out + (size_t)(tok0 + c0) * P.ldc + orow;
+        const int live = orow < P.n ? min(16, P.m - tok0 - c0) : 0;
+        // the old values of an accumulating product are loaded together, in front of the first store: written as one
+        // read-modify-write after the other they were sixteen round trips to L2 in a row
+        float old[16];
+        if (P.accumulate) {
+#pragma unroll
+          for (int w = 0; w < 16; ++w) old[w] = w < live ? __ldcg(dst + (size_t)w * P.ldc) : 0.0f;
+        }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int w = 0; w < 16; ++w) {
-          const int tok = tok0 + c0 + w;
-          if (tok < P.m && orow < P.n) {
-            float *dst = out + (size_t)tok * P.ldc + orow;
-            *dst = P.accumulate ? __fadd_rn(*dst, __uint_as_float(v[w])) : __uint_as_float(v[w]);
-          }
+          const float x = __uint_as_float(v[w]);
+          if (w < live) dst[(size_t)w * P.ldc] = P.accumulate ? __fadd_rn(old[w], x) : x;
         }
       }
     }
@@ -449,7 +538,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(T::TMEM_COLS) : "memory");
   }
 }
 
@@ -470,13 +559,11 @@ EncodeFn encode_fn() {
 
 template <int QT, int TN, int MODE, int RT>
 cudaError_t launch_t(const QGemmArgs &a, const LaunchCfg &cfg) {
+  using T = Tile<QT, TN, MODE, RT>;
   EncodeFn fn = encode_fn();
   if (!fn) return cudaErrorNotSupported;
-  constexpr bool F16 = MODE != QGEMM_BF16, COMP = MODE == QGEMM_F16X3;
-  constexpr int BB = (QT == RG_TYPE_Q4_0) ? 18 : 34;
-  constexpr int NS = ring_depth(TN, COMP);
-  constexpr int NPL = COMP ? 2 : 1;
-  constexpr int RAW_ROW = 8 * BB;
+  constexpr bool F16 = T::F16, COMP = T::COMP;
+  constexpr int BB = T::BB, NPL = T::NPL, RAW_ROW = T::RAW_ROW;
   alignas(64) CUtensorMap xmap, xlo_map, wmap;
   const cuuint32_t elem[2] = {1, 1};
   for (int plane = 0; plane < NPL; ++plane) {
@@ -513,20 +600,18 @@ cudaError_t launch_t(const QGemmArgs &a, const LaunchCfg &cfg) {
   P.status = cfg.status;
   P.accumulate = a.accumulate ? 1 : 0;
   if (a.accumulate && splits > 1) return cudaErrorInvalidValue;
-  constexpr size_t smem = 1024 + NS * NPL * (TN * KSTEP * 2) + RAW_NS * RT * TM * RAW_ROW + (3 * NS + 2 * RAW_NS + 1) * 8 + 16;
-  static_assert(smem <= 227 * 1024, "tile configuration exceeds the shared memory of one SM");
   auto kernel = qgemm_tc_kernel<QT, TN, MODE, RT>;
   static DeviceOnce attr_once;  // per instantiation and device
   bool *attr_flag = attr_once.slot();
   if (!attr_flag || !*attr_flag) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     if (attr_flag) *attr_flag = true;
   }
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3((unsigned)((a.n + TM * RT - 1) / (TM * RT)), (unsigned)((a.m + TN - 1) / TN), (unsigned)splits);
-  lc.blockDim = dim3(64 + RT * 256);
-  lc.dynamicSmemBytes = smem;
+  lc.blockDim = dim3(T::THREADS);
+  lc.dynamicSmemBytes = T::SMEM_BYTES;
   lc.stream = cfg.stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -536,17 +621,50 @@ cudaError_t launch_t(const QGemmArgs &a, const LaunchCfg &cfg) {
   return cudaLaunchKernelEx(&lc, kernel, xmap, xlo_map, wmap, P);
 }
 
+// Tile of a compensated product.  Whatever the tile, an output's products are added in the same order, so the choice
+// moves no bit.  A step of 64 elements costs a CTA at least its MMAs (12 a row tile, 14 to 64 cycles each by the tile's width), and
+// narrow tiles the dequantisation they repeat per token tile; what else is lost is the last wave of CTAs.  The estimate
+// is the measured time of a tile with K = 4096 (in units of 0.1 us): `solo` when the grid leaves no SM with two, else `wave` for
+// every whole wave of the SMs.  The earlier entry wins a tie.  [4096, 4096] x 117 tokens: 63.7 us in 2 x 128 tiles of 128 tokens,
+// 39 / 31 / 29 in tiles of 128 / 64 / 32 (72 before); [28672, 4096] x 1024: 494 / 482 / 573 / 830 (550 before).
+struct TileCost {
+  int rt, tn, solo, wave;
+};
+constexpr TileCost TILES_Q4[] = {{2, 128, 650, 700}, {1, 128, 395, 370}, {1, 64, 315, 245}, {1, 32, 290, 200}, {1, 16, 280, 190}};
+constexpr TileCost TILES_Q8[] = {{2, 128, 710, 795}, {1, 128, 435, 460}, {1, 64, 400, 345}, {1, 32, 395, 310}, {1, 16, 390, 300}};
+template <int QT>
+TileCost tile_of(const QGemmArgs &a, int sm_count) {
+  TileCost best{0, 0, 0, 0};
+  long best_cost = 0;
+  for (const TileCost &t : QT == RG_TYPE_Q4_0 ? TILES_Q4 : TILES_Q8) {
+    const long tiles = (long)((a.n + TM * t.rt - 1) / (TM * t.rt)) * ((a.m + t.tn - 1) / t.tn) * (a.splits > 1 ? a.splits : 1);
+    const long waves = (tiles + sm_count - 1) / sm_count, cost = waves == 1 ? t.solo : waves * t.wave;
+    if (!best.rt || cost < best_cost) {
+      best = t;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 template <int QT, int MODE>
 cudaError_t launch_n(const QGemmArgs &a, const LaunchCfg &cfg) {
-  constexpr int RT = row_tiles(MODE);
-  // accumulators (RT tiles of TN columns) and the A ring share the 512 columns of tensor memory
-  if constexpr (RT == 1) {
-    if (a.m > 128) return launch_t<QT, 256, MODE, RT>(a, cfg);
+  if constexpr (MODE == QGEMM_F16X3) {
+    const TileCost t = tile_of<QT>(a, cfg.sm_count > 0 ? cfg.sm_count : 148);
+    if (t.rt == 2) return launch_t<QT, 128, MODE, 2>(a, cfg);
+    switch (t.tn) {
+      case 128: return launch_t<QT, 128, MODE, 1>(a, cfg);
+      case 64: return launch_t<QT, 64, MODE, 1>(a, cfg);
+      case 32: return launch_t<QT, 32, MODE, 1>(a, cfg);
+      default: return launch_t<QT, 16, MODE, 1>(a, cfg);
+    }
+  } else {
+    if (a.m > 128) return launch_t<QT, 256, MODE, 1>(a, cfg);
+    if (a.m > 64) return launch_t<QT, 128, MODE, 1>(a, cfg);
+    if (a.m > 32) return launch_t<QT, 64, MODE, 1>(a, cfg);
+    if (a.m > 16) return launch_t<QT, 32, MODE, 1>(a, cfg);
+    return launch_t<QT, 16, MODE, 1>(a, cfg);
   }
-  if (a.m > 64) return launch_t<QT, 128, MODE, RT>(a, cfg);
-  if (a.m > 32) return launch_t<QT, 64, MODE, RT>(a, cfg);
-  if (a.m > 16) return launch_t<QT, 32, MODE, RT>(a, cfg);
-  return launch_t<QT, 16, MODE, RT>(a, cfg);
 }
 template <int QT>
 cudaError_t launch_m(const QGemmArgs &a, const LaunchCfg &cfg) {
@@ -684,7 +802,7 @@ static int effective_splits(int k, int splits) {
 // chunk.
 int qgemm_splits(int n, int k, int m, int mode, int sm_count, size_t scratch_floats) {
   if (m > QGEMM_SPLIT_MAX_TOKENS || k < KSTEP * RAW_STEPS) return 1;
-  const int rows = TM * row_tiles(mode), tiles = (n + rows - 1) / rows;
+  const int rows = TM * (mode == QGEMM_F16X3 ? 2 : 1), tiles = (n + rows - 1) / rows;
   int splits = effective_splits(k, 2 * sm_count / tiles);
   while (splits > 1 && (size_t)splits * (size_t)m * (size_t)n > scratch_floats) --splits;
   return effective_splits(k, splits);  // the launcher's own count: the reduction sums exactly the tiles it writes

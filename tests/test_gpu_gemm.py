@@ -138,3 +138,20 @@ def test_prefill_shapes_below_the_wide_tile_threshold(m, n, k):
     want = x.astype(np.float64) @ dense.T
     scale = np.sqrt((x.astype(np.float64) ** 2).sum(1))[:, None] * np.sqrt((dense ** 2).sum(1))[None, :]
     assert (np.abs(got - want) / scale).max() < 2e-6
+
+
+@pytest.mark.parametrize("kind", [quant.Q4_0, quant.Q8_0])
+@pytest.mark.parametrize("n,k", [(1, 256), (127, 512), (129, 1280), (700, 768), (20000, 256)])
+def test_a_row_of_a_compensated_product_does_not_depend_on_its_tile(kind, n, k):
+    """Tiles of 16 to 128 tokens and of one or two row tiles add up the products of an output in the same order, so an
+    activation row gives the same bits in products of any number of rows; edges of every tile width and of the weight rows.
+    Bound: f32 accumulation, 2e-6 of the norms."""
+    rng = np.random.default_rng(n + k)
+    data = quant.encode(kind, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = rng.standard_normal((300, k), dtype=np.float32)
+    dense = O.dequantize(kind, data, n * k).reshape(n, k).astype(np.float64)
+    whole, _ = session.qgemm(kind, data, n, k, x, operand_mode=2)
+    scale = np.sqrt((x.astype(np.float64) ** 2).sum(1))[:, None] * np.sqrt((dense ** 2).sum(1))[None, :]
+    assert (np.abs(whole - x.astype(np.float64) @ dense.T) / scale).max() < 2e-6
+    for m in (1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 257):
+        np.testing.assert_array_equal(session.qgemm(kind, data, n, k, x[:m], operand_mode=2)[0], whole[:m])
