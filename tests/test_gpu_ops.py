@@ -204,6 +204,25 @@ def test_decode_attention_rejects_unsupported_head_geometry():
     assert e.value.status == 20
 
 
+@pytest.mark.parametrize("kind", [quant.Q4_0, quant.Q8_0])
+@pytest.mark.parametrize("n,k", [(1, 256), (40, 512), (257, 2048), (1000, 7168)])
+def test_batch_gemv_at_the_edges_of_its_column_tiles(kind, n, k):
+    """Both sides of every count of column tiles (four rows each).  A row's sums do not depend on the count of tiles beside its own
+    chunk length: 5 to 16 rows share one.  Bound: 22-bit activations and f32 sums, 1e-6 of the norms."""
+    rng = np.random.default_rng(n * 3 + k)
+    data = quant.encode(kind, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    x = rng.standard_normal((16, k), dtype=np.float32)
+    dense = O.dequantize(kind, data, n * k).reshape(n, k).astype(np.float64)
+    scale = np.sqrt((x.astype(np.float64) ** 2).sum(1))[:, None] * np.sqrt((dense ** 2).sum(1))[None, :]
+    whole = session.qmatmul(kind, data, n, k, x)
+    for m in (3, 4, 5, 8, 9, 11, 12, 13, 16):
+        got = session.qmatmul(kind, data, n, k, x[:m])
+        assert (np.abs(got - x[:m].astype(np.float64) @ dense.T) / scale[:m]).max() < 1e-6
+        if m >= 5:
+            np.testing.assert_array_equal(got, whole[:m])
+
+
+
 def test_opt_in_row_gemv_matches_f64_blockwise_plan():
     """The second 3..16-row GEMV (qgemv_rows.cu, switched on by RG_B200_ROWS_GEMV=1 when the library
     loads, hence the child process): tall row tiles, K split over CTAs for matrices with few rows and
