@@ -201,6 +201,19 @@ struct TpFusedArgs {
 constexpr int TP_PUSH_COLS = 32;  // columns an exchange in push form can carry
 cudaError_t launch_tp_allreduce_add(const TpFusedArgs &a, const LaunchCfg &cfg);
 
+// Cached positions of one row copied between the caches of up to KV_COPY_MAX (layer, K or V) pairs and a packed block:
+// for every pair and kv head, `bytes` consecutive bytes.  Offsets, pitches and sizes are multiples of 16 bytes.
+constexpr int KV_COPY_MAX = 128;
+struct KvCopyArgs {
+  uint8_t *cache[KV_COPY_MAX];  // first byte of the row in each cache
+  size_t cache_pitch = 0;       // kv head to kv head
+  uint8_t *packed = nullptr;    // [pair][kv head][bytes]
+  size_t bytes = 0;
+  int pairs = 0, kv_heads = 0;
+  bool to_cache = false;
+};
+cudaError_t launch_kv_copy(const KvCopyArgs &a, cudaStream_t stream);
+
 // Dense (F32/F16) weight GEMV for tensors the block formats cannot hold (K % 32 != 0) or that a
 // file stores dense.  x is plain f32 [batch, ldx]; same epilogues (EPI_SWIGLU unsupported).
 struct DenseGemvArgs {

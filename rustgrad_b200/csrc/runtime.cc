@@ -2447,6 +2447,28 @@ struct rg_kv_snapshot {
 
 static size_t kv_esize(const rg_session *s) { return s->kv_f32 ? 4 : 2; }
 
+// Copies `length` positions of cache row `row` of every layer into the snapshot's block or back.
+static cudaError_t kv_copy(rg_session *s, const rg_kv_snapshot *k, int32_t row, bool to_cache) {
+  KvCopyArgs a;
+  a.cache_pitch = (size_t)s->ctx * (size_t)s->cfg.head_dim * kv_esize(s);
+  a.bytes = k->row_bytes;
+  a.kv_heads = k->kv_heads;
+  a.to_cache = to_cache;
+  const size_t row_off = (size_t)row * (size_t)k->kv_heads * a.cache_pitch;
+  const int pairs = 2 * k->n_layers;
+  for (int p0 = 0; p0 < pairs; p0 += KV_COPY_MAX) {
+    a.pairs = std::min(KV_COPY_MAX, pairs - p0);
+    for (int i = 0; i < a.pairs; ++i) {
+      const size_t l = (size_t)(p0 + i) / 2;
+      a.cache[i] = static_cast<uint8_t *>(((p0 + i) & 1) ? s->v_cache[l] : s->k_cache[l]) + row_off;
+    }
+    a.packed = k->data + (size_t)p0 * (size_t)k->kv_heads * k->row_bytes;
+    const cudaError_t e = launch_kv_copy(a, s->stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 int32_t rg_b200_kv_snapshot_create(rg_session *s, int32_t row, int32_t length, rg_kv_snapshot **out) {
   int32_t rc = check_live(s);
   if (rc) return rc;
@@ -2464,20 +2486,12 @@ int32_t rg_b200_kv_snapshot_create(rg_session *s, int32_t row, int32_t length, r
   void *p = nullptr;
   if (x_malloc(&p, snap->bytes) != cudaSuccess) return fail(RG_OUT_OF_MEMORY, "KV snapshot of " + std::to_string(snap->bytes) + " bytes");
   snap->data = static_cast<uint8_t *>(p);
-  const size_t src_pitch = (size_t)s->ctx * hd * es, head_block = (size_t)snap->kv_heads * snap->row_bytes;
-  for (int l = 0; l < snap->n_layers; ++l)
-    for (int kv = 0; kv < 2; ++kv) {
-      const uint8_t *src = static_cast<const uint8_t *>(kv ? s->v_cache[(size_t)l] : s->k_cache[(size_t)l]) +
-                           (size_t)row * (size_t)snap->kv_heads * src_pitch;
-      uint8_t *dst = snap->data + ((size_t)l * 2 + (size_t)kv) * head_block;
-      cudaError_t e = cudaMemcpy2DAsync(dst, snap->row_bytes, src, src_pitch, snap->row_bytes, (size_t)snap->kv_heads,
-                                        cudaMemcpyDeviceToDevice, s->stream);
-      if (e != cudaSuccess) {
-        cudaFree(snap->data);
-        return fail(RG_CUDA_ERROR, std::string("snapshot copy: ") + cudaGetErrorString(e));
-      }
-    }
-  cudaError_t e = x_sync(s->stream);
+  cudaError_t e = kv_copy(s, snap.get(), row, false);
+  if (e != cudaSuccess) {
+    cudaFree(snap->data);
+    return fail(RG_CUDA_ERROR, std::string("snapshot copy: ") + cudaGetErrorString(e));
+  }
+  e = x_sync(s->stream);
   if (e != cudaSuccess) {
     cudaFree(snap->data);
     s->poisoned = true;
@@ -2499,13 +2513,7 @@ int32_t rg_b200_kv_snapshot_restore(rg_session *s, const rg_kv_snapshot *k, int3
       k->row_bytes != (size_t)k->length * hd * es)
     return fail(RG_SHAPE_MISMATCH, "snapshot was taken from a session of another shape");
   RG_CUDA(cudaSetDevice(s->opt.device));
-  const size_t dst_pitch = (size_t)s->ctx * hd * es, head_block = (size_t)k->kv_heads * k->row_bytes;
-  for (int l = 0; l < k->n_layers; ++l)
-    for (int kv = 0; kv < 2; ++kv) {
-      uint8_t *dst = static_cast<uint8_t *>(kv ? s->v_cache[(size_t)l] : s->k_cache[(size_t)l]) + (size_t)row * (size_t)k->kv_heads * dst_pitch;
-      const uint8_t *src = k->data + ((size_t)l * 2 + (size_t)kv) * head_block;
-      RG_CUDA(cudaMemcpy2DAsync(dst, dst_pitch, src, k->row_bytes, k->row_bytes, (size_t)k->kv_heads, cudaMemcpyDeviceToDevice, s->stream));
-    }
+  RG_CUDA(kv_copy(s, k, row, true));
   cudaError_t e = x_sync(s->stream);
   if (e != cudaSuccess) {
     s->poisoned = true;
