@@ -2,6 +2,7 @@
 // RoPE + KV append, split-context GQA attention + combine, greedy selection, dense-weight GEMV,
 // and the synthetic-tensor generator.  All are HBM/latency-bound SIMT kernels; each calls
 // pdl_wait() before touching step data so programmatic dependent launch stays transitive.
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <mutex>
@@ -1140,10 +1141,228 @@ cudaError_t launch_fill_f32(float *out, size_t n, float v, const LaunchCfg &cfg)
 //    (different streams without an ordering between them) race on it; order them.  Nothing in
 //    the array has to start at zero: each call overwrites every partial it later reads, and the
 //    three control words in front of the partials are rewritten by a kernel at the start of each call.
+//    (Up to CL_MAX_POS positions only a waiting call touches the array: its status word.)
 namespace {
 constexpr size_t NOALLOC_SCRATCH_FLOATS = size_t(1) << 20;
 constexpr size_t NOALLOC_HEADER_FLOATS = 64;  // control words: sequence, position, status
 static __device__ __align__(256) float g_noalloc_attn[NOALLOC_HEADER_FLOATS + NOALLOC_SCRATCH_FLOATS];
+
+// One launch for the whole attention: a cluster of eight CTAs owns a kv head, every CTA an eighth of the positions in
+// tiles of 64 KB of K and V rows (double-buffered bulk copies), and the cluster merges its eight partial results through
+// distributed shared memory, so no partial goes through memory and no second kernel waits for the first.
+// Bound by latency: the score and P.V loops of one CTA's positions.  32 heads over 8 kv heads, f16, in a captured graph: 16 / 512 / 2048
+// positions 6.6 / 11.1 / 16.2 -> 5.5 / 6.8 / 12.5 us; called one after the other at 2048, where the host's three launches
+// counted, 21.5 -> 14.4.
+constexpr int CL_CTAS = 8;
+constexpr int CL_TILE_BYTES = 32 * 1024;  // of K, and as much of V
+// sixteen warps where the registers of the G heads allow it
+template <int G>
+constexpr int CL_THREADS = G == 8 ? 256 : 512;
+constexpr int CL_SMEM = 2 * 2 * CL_TILE_BYTES + 128;
+
+template <typename KV, int G, int HD>
+__global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_THREADS<G>)
+    attn_cluster_kernel(const float *q, const KV *k_cache, const KV *v_cache, int ctx, int n_pos, float *out, int *status) {
+  constexpr int TILE = CL_TILE_BYTES / (HD * (int)sizeof(KV));  // positions of a tile: 64 .. 256
+  constexpr int THREADS = CL_THREADS<G>, WARPS = THREADS / 32;
+  constexpr int DPL = HD / 16;  // dims per lane, scores
+  constexpr int DV = HD / 32;   // dims per lane, P.V
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), kvh = blockIdx.y;
+  // positions of each CTA: an eighth, in whole units of 16 (one pass of the score loop)
+  const int per = ((n_pos + CL_CTAS - 1) / CL_CTAS + 15) & ~15;
+  const int p0 = min(n_pos, rank * per), p1 = min(n_pos, p0 + per);
+  const int n_tiles = (p1 - p0 + TILE - 1) / TILE;
+
+  __shared__ __align__(16) float sc[TILE][G];
+  __shared__ float m_run[G], l_run[G], corr[G];
+  __shared__ __align__(16) float part[G][HD];  // this CTA's sum of P.V, read by the whole cluster
+  __shared__ __align__(8) uint64_t bars[4];    // K and V of either buffer
+  __shared__ int dead_flag;
+  extern __shared__ __align__(128) uint8_t att_smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int i = 0; i < 4; ++i) mbar_init(&bars[i], 1);
+    dead_flag = 0;
+    mbar_fence_init();
+  }
+  if (tid < G) {
+    m_run[tid] = -INFINITY;
+    l_run[tid] = 0.0f;
+  }
+  __syncthreads();
+  const KV *kg = k_cache + (size_t)kvh * ctx * HD, *vg = v_cache + (size_t)kvh * ctx * HD;
+  auto issue = [&](int t) {  // thread 0
+    const int buf = t & 1, first = p0 + t * TILE, np = min(TILE, p1 - first);
+    const uint32_t bytes = (uint32_t)(np * HD * (int)sizeof(KV));
+    uint8_t *dst = att_smem + buf * 2 * CL_TILE_BYTES;
+    mbar_expect_tx(&bars[2 * buf], bytes);
+    bulk_g2s(dst, kg + (size_t)first * HD, bytes, &bars[2 * buf]);
+    mbar_expect_tx(&bars[2 * buf + 1], bytes);
+    bulk_g2s(dst + CL_TILE_BYTES, vg + (size_t)first * HD, bytes, &bars[2 * buf + 1]);
+  };
+  if (tid == 0) {
+    if (n_tiles > 0) issue(0);
+    if (n_tiles > 1) issue(1);
+  }
+  const float inv_scale = (float)(1.0 / (1.0 / sqrt((double)HD)));
+  const int sub = lane & 15, hi = lane >> 4;
+  float qr[G][DPL];
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) qr[g][i] = q[((size_t)kvh * G + g) * HD + sub * DPL + i];
+  float acc[G][DV];
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int i = 0; i < DV; ++i) acc[g][i] = 0.0f;
+
+  for (int t = 0; t < n_tiles; ++t) {
+    const int buf = t & 1, np = min(TILE, p1 - p0 - t * TILE);
+    const uint32_t phase = (uint32_t)((t >> 1) & 1);
+    const KV *ks = reinterpret_cast<const KV *>(att_smem + buf * 2 * CL_TILE_BYTES);
+    const KV *vs = reinterpret_cast<const KV *>(att_smem + buf * 2 * CL_TILE_BYTES + CL_TILE_BYTES);
+    mbar_wait_bounded(&bars[2 * buf], phase, &dead_flag, status);
+    for (int base = 0; base < np; base += 2 * WARPS) {
+      const int p = base + warp * 2 + hi;
+      float kv[DPL];
+      if (p < np) {
+        kv_load_vec<DPL>(ks + (size_t)p * HD + sub * DPL, kv);
+      } else {
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) kv[i] = 0.0f;
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        float dot = 0.0f;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) dot = fmaf(qr[g][i], kv[i], dot);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (sub == 0 && p < np) sc[p][g] = __fdiv_rn(dot, inv_scale);
+      }
+    }
+    __syncthreads();
+    if (warp < G) {
+      const int g = warp;
+      float m = m_run[g];
+      const float before = m;
+      for (int p = lane; p < np; p += 32) m = fmaxf(m, sc[p][g]);
+      m = warp_max(m);
+      float l = 0.0f;
+      for (int p = lane; p < np; p += 32) {
+        const float e = exp2f(__fmul_rn(__fsub_rn(sc[p][g], m), 1.44269504088896340736f));
+        sc[p][g] = e;
+        l += e;
+      }
+      l = warp_sum(l);
+      if (lane == 0) {
+        // nothing has been summed before the first tile, whose maximum may itself be -inf
+        const float c = t == 0 ? 0.0f : exp2f(__fmul_rn(__fsub_rn(before, m), 1.44269504088896340736f));
+        corr[g] = c;
+        m_run[g] = m;
+        l_run[g] = t == 0 ? l : fmaf(l_run[g], c, l);
+      }
+    }
+    __syncthreads();
+    mbar_wait_bounded(&bars[2 * buf + 1], phase, &dead_flag, status);
+    if (t > 0) {
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int i = 0; i < DV; ++i) acc[g][i] *= corr[g];
+    }
+#pragma unroll 4
+    for (int p = warp; p < np; p += WARPS) {
+      float v[DV];
+      kv_load_vec<DV>(vs + (size_t)p * HD + lane * DV, v);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const float pr = sc[p][g];
+#pragma unroll
+        for (int i = 0; i < DV; ++i) acc[g][i] = fmaf(pr, v[i], acc[g][i]);
+      }
+    }
+    __syncthreads();  // everyone is done with the buffer and with the scores
+    if (tid == 0 && t + 2 < n_tiles) issue(t + 2);
+  }
+  // the warps' sums of P.V, in warp order (the tile buffers are free: every copy has been waited for)
+  float *red = reinterpret_cast<float *>(att_smem);  // [warp][G][HD]
+  static_assert(WARPS * G * HD * 4 <= 4 * CL_TILE_BYTES, "the sums reuse the tile buffers");
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int i = 0; i < DV; ++i) red[(warp * G + g) * HD + lane * DV + i] = acc[g][i];
+  __syncthreads();
+  for (int idx = tid; idx < G * HD; idx += THREADS) {
+    float v = 0.0f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) v += red[w * G * HD + idx];
+    part[idx / HD][idx % HD] = v;
+  }
+  cluster.sync();
+  // every CTA finishes an eighth of the kv head's G * HD outputs, from the CTAs that hold positions, in order
+  const int n_live = (n_pos + per - 1) / per;
+  constexpr int MINE = G * HD / CL_CTAS;
+  if (tid < MINE) {
+    const int idx = rank * MINE + tid, g = idx / HD, d = idx - g * HD;
+    float ms[CL_CTAS], ls[CL_CTAS], vs[CL_CTAS];
+#pragma unroll
+    for (int r = 0; r < CL_CTAS; ++r)
+      if (r < n_live) {
+        ms[r] = *cluster.map_shared_rank(&m_run[g], r);
+        ls[r] = *cluster.map_shared_rank(&l_run[g], r);
+        vs[r] = *cluster.map_shared_rank(&part[g][d], r);
+      }
+    float M = -INFINITY, L = 0.0f, v = 0.0f;
+#pragma unroll
+    for (int r = 0; r < CL_CTAS; ++r)
+      if (r < n_live) M = fmaxf(M, ms[r]);
+#pragma unroll
+    for (int r = 0; r < CL_CTAS; ++r)
+      if (r < n_live) {
+        const float wgt = exp2f(__fmul_rn(__fsub_rn(ms[r], M), 1.44269504088896340736f));
+        L = fmaf(ls[r], wgt, L);
+        v = fmaf(vs[r], wgt, v);
+      }
+    out[((size_t)kvh * G + g) * HD + d] = __fmul_rn(v, __frcp_rn(L));
+  }
+  cluster.sync();  // no CTA leaves while another may still read its shared memory
+}
+
+// The one-launch form is taken up to this many positions: eight CTAs a kv head are few for long contexts.  Calls in a row / in a graph, us,
+// new against three launches: 3000 positions 18.6 / 16.6 and 24.2 / 17.8; 4096 22.7 / 20.7 and 24.8 / 19.7; 8000 (two kv heads)
+// 39.0 / 36.8 and 31.9 / 27.0.
+constexpr int CL_MAX_POS = 4096;
+
+template <typename KV, int G, int HD>
+cudaError_t launch_attn_cluster_t(const float *q, const void *k, const void *v, int kv_heads, int ctx, int n_pos, float *out, int *status,
+                                  cudaStream_t st) {
+  auto kernel = attn_cluster_kernel<KV, G, HD>;
+  static DeviceOnce attr_once;  // per instantiation and device
+  bool *attr_flag = attr_once.slot();
+  if (!attr_flag || !*attr_flag) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CL_SMEM);
+    if (e != cudaSuccess) return e;
+    if (attr_flag) *attr_flag = true;
+  }
+  kernel<<<dim3(CL_CTAS, (unsigned)kv_heads), CL_THREADS<G>, CL_SMEM, st>>>(q, static_cast<const KV *>(k), static_cast<const KV *>(v), ctx, n_pos,
+                                                                         out, status);
+  return cudaGetLastError();
+}
+template <typename KV, int HD>
+cudaError_t launch_attn_cluster(const float *q, const void *k, const void *v, int heads, int kv_heads, int ctx, int n_pos, float *out,
+                                int *status, cudaStream_t st) {
+  switch (heads / kv_heads) {
+    case 1: return launch_attn_cluster_t<KV, 1, HD>(q, k, v, kv_heads, ctx, n_pos, out, status, st);
+    case 2: return launch_attn_cluster_t<KV, 2, HD>(q, k, v, kv_heads, ctx, n_pos, out, status, st);
+    case 4: return launch_attn_cluster_t<KV, 4, HD>(q, k, v, kv_heads, ctx, n_pos, out, status, st);
+    case 8: return launch_attn_cluster_t<KV, 8, HD>(q, k, v, kv_heads, ctx, n_pos, out, status, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 __global__ void noalloc_header_kernel(int32_t *header, int32_t pos) {
   header[0] = 0;    // the single sequence
@@ -1205,27 +1424,41 @@ extern "C" int32_t rg_b200_attention_decode_noalloc(const float *q_dev, const vo
   if (e != cudaSuccess) return fail(RG_CUDA_ERROR, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
   int32_t *header = reinterpret_cast<int32_t *>(base);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  noalloc_header_kernel<<<1, 1, 0, st>>>(header, n_pos - 1);
-  if ((e = cudaGetLastError()) != cudaSuccess) return fail(RG_CUDA_ERROR, std::string("header launch: ") + cudaGetErrorString(e));
-  LaunchCfg cfg;
-  cfg.stream = st;
-  cfg.pdl = false;
-  cfg.status = header + 2;
-  AttnArgs a;
-  a.q = q_dev;
-  a.k_cache = keys_dev;
-  a.v_cache = values_dev;
-  a.kv_f32 = kv_f32 != 0;
-  a.cols = 1;
-  a.heads = heads;
-  a.kv_heads = kv_heads;
-  a.hd = head_dim;
-  a.ctx = ctx;
-  a.col_seq = header;
-  a.col_pos = header + 1;
-  a.scratch = base + NOALLOC_HEADER_FLOATS;
-  a.out_f32 = out_dev;
-  if ((e = launch_attention(a, cfg)) != cudaSuccess) return fail(RG_CUDA_ERROR, std::string("attention launch: ") + cudaGetErrorString(e));
+  if (n_pos <= CL_MAX_POS) {
+    // the status word is only ever read by a waiting call, so only that one clears it first
+    if (wait && (e = cudaMemsetAsync(header + 2, 0, sizeof(int32_t), st)) != cudaSuccess)
+      return fail(RG_CUDA_ERROR, std::string("status reset: ") + cudaGetErrorString(e));
+    count_launch(LC_ATTN_SPLIT);
+    if (kv_f32)
+      e = head_dim == 128 ? launch_attn_cluster<float, 128>(q_dev, keys_dev, values_dev, heads, kv_heads, ctx, n_pos, out_dev, header + 2, st)
+                          : launch_attn_cluster<float, 64>(q_dev, keys_dev, values_dev, heads, kv_heads, ctx, n_pos, out_dev, header + 2, st);
+    else
+      e = head_dim == 128 ? launch_attn_cluster<__half, 128>(q_dev, keys_dev, values_dev, heads, kv_heads, ctx, n_pos, out_dev, header + 2, st)
+                          : launch_attn_cluster<__half, 64>(q_dev, keys_dev, values_dev, heads, kv_heads, ctx, n_pos, out_dev, header + 2, st);
+    if (e != cudaSuccess) return fail(RG_CUDA_ERROR, std::string("attention launch: ") + cudaGetErrorString(e));
+  } else {
+    noalloc_header_kernel<<<1, 1, 0, st>>>(header, n_pos - 1);
+    if ((e = cudaGetLastError()) != cudaSuccess) return fail(RG_CUDA_ERROR, std::string("header launch: ") + cudaGetErrorString(e));
+    LaunchCfg cfg;
+    cfg.stream = st;
+    cfg.pdl = false;
+    cfg.status = header + 2;
+    AttnArgs a;
+    a.q = q_dev;
+    a.k_cache = keys_dev;
+    a.v_cache = values_dev;
+    a.kv_f32 = kv_f32 != 0;
+    a.cols = 1;
+    a.heads = heads;
+    a.kv_heads = kv_heads;
+    a.hd = head_dim;
+    a.ctx = ctx;
+    a.col_seq = header;
+    a.col_pos = header + 1;
+    a.scratch = base + NOALLOC_HEADER_FLOATS;
+    a.out_f32 = out_dev;
+    if ((e = launch_attention(a, cfg)) != cudaSuccess) return fail(RG_CUDA_ERROR, std::string("attention launch: ") + cudaGetErrorString(e));
+  }
   if (wait) {
     int status = 0;
     if ((e = cudaMemcpyAsync(&status, header + 2, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||

@@ -84,3 +84,26 @@ def test_sizes_beyond_the_fixed_array_are_refused():
     assert L.rg_b200_attention_decode_noalloc(p, p, odd, 8, 2, 128, 64, 1, 0, p, None, 1) == 1
     assert b"16-byte" in L.rg_b200_last_error()
     assert L.rg_b200_attention_decode_noalloc(C.c_void_p(buf.data_ptr() + 2), p, p, 8, 2, 128, 64, 1, 0, p, None, 1) == 1
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd", [(4, 4, 64), (4, 2, 128), (8, 2, 64), (16, 2, 128)])
+@pytest.mark.parametrize("dtype", [np.float16, np.float32])
+def test_positions_at_the_edges_of_the_cluster_split(heads, kv_heads, hd, dtype):
+    """One position to eight CTAs with several tiles each, both sides of every unit of 16 and of the longest context the one-launch form
+    takes.  Both entry points sum in f32 in different orders: 2^-24 of values of a few units times the square root of a few dozen sums."""
+    for n_pos in (1, 15, 16, 17, 127, 128, 129, 511, 513, 1024, 1025, 2049, 4096, 4097):
+        q, k, v = case(n_pos, heads, kv_heads, hd, n_pos, dtype)
+        want = session.attention_decode(q, k, v)
+        got = run_noalloc(q, k, v, n_pos + 3)
+        assert np.abs(got - want).max() <= 2e-6, n_pos
+
+
+def test_special_values_pass_through_as_in_the_ordinary_entry_point():
+    """Scores of -inf leave no weight (a tile of nothing else gives NaN), NaN and +inf reach the output."""
+    for where, value in ((5, -np.inf), (200, np.inf), (299, np.nan)):
+        q, k, v = case(9, 4, 2, 128, 300, np.float16)
+        k[0, where, :] = value
+        want, got = session.attention_decode(q, k, v), run_noalloc(q, k, v, 320)
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+        fine = ~np.isnan(want)
+        assert np.abs(got[fine] - want[fine]).max(initial=0.0) <= 2e-6
