@@ -12,8 +12,12 @@
 //  * online softmax per warp (exp2 form, running max / sum);
 //  * O += P V with P as hi + lo planes straight from the score accumulators, V read transposed by
 //    ldmatrix.
-// The four warps' (max, sum, O) merge in shared memory into one partial result of the span, and a
-// second small kernel merges the spans of a head in span order.  Every f16 x f16 product is exact in
+// The four warps' (max, sum, O) merge in shared memory into one partial result of the span.  Where a (row, kv head) has at
+// most eight spans its CTAs are a cluster: every CTA rotates the query itself out of the raw projections, the one with
+// the last span also rotates and appends the new K / V row (and multiplies it out of shared memory), and the spans merge
+// through distributed shared memory in span order: one launch instead of three (16 rows of the 8B shape behind 2100
+// positions: 1.35 -> 1.25 ms a step).  With
+// more spans a second small kernel merges them, behind rope_append.  Every f16 x f16 product is exact in
 // the f32 accumulator; what differs from the f32 kernels is the order of the sums and the 2^-22 tail
 // of q and p.
 #include <cuda_fp16.h>
@@ -39,8 +43,11 @@ constexpr int MAX_G = 8;
 constexpr int Q_BYTES = 2 * 16 * LD * 2;                    // hi and lo plane of the 16-row query tile
 constexpr int STAGE_BYTES = 2 * TK * LD * 2;                // K tile + V tile
 constexpr int RING_BYTES = WARPS * NSTG * STAGE_BYTES;
-constexpr int SMEM_BYTES = Q_BYTES + RING_BYTES;
-static_assert(WARPS * MAX_G * (HD + 2) * 4 <= RING_BYTES, "the merge buffer reuses the ring");
+constexpr int NEW_BYTES = 2 * HD * 2;                       // the row's new K and V (fused form)
+constexpr int SMEM_BYTES = Q_BYTES + RING_BYTES + NEW_BYTES;
+constexpr int MERGE_FLOATS = WARPS * MAX_G * (HD + 2);
+static_assert((MERGE_FLOATS + MAX_G * (HD + 2)) * 4 <= RING_BYTES, "the merge buffers reuse the ring");
+constexpr int MAX_CLUSTER = 8;
 
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
@@ -81,7 +88,19 @@ __host__ __device__ inline int span_len(int total, int per_head) {
   return span < SPAN_UNIT ? SPAN_UNIT : span;
 }
 
-template <int G>
+__device__ __forceinline__ float ld_cluster(const float *local, int rank) {
+  uint32_t remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// FUSED: gridDim.x = cluster size = per_head
+template <int G, bool FUSED>
 __global__ void __launch_bounds__(THREADS, 2) attn_decode_tc_kernel(const AttnArgs A, int per_head) {
   pdl_wait();
   pdl_launch_dependents();
@@ -90,26 +109,58 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_tc_kernel(const AttnAr
   const int total = pos + 1;
   const int span = span_len(total, per_head);
   const int nspl = (total + span - 1) / span;
-  if (sp >= nspl) return;
-  const int p0 = sp * span, p1 = min(total, p0 + span);
+  if (!FUSED && sp >= nspl) return;
+  const int p0 = min(total, sp * span), p1 = min(total, p0 + span);  // a CTA of a cluster may have no keys
+  const bool has_new = FUSED && p1 == total && p0 < p1;              // the new token's own position
 
   extern __shared__ __align__(16) uint8_t smem[];
   __half *q_hi = reinterpret_cast<__half *>(smem);  // [16][LD]
   __half *q_lo = q_hi + 16 * LD;
   uint8_t *ring = smem + Q_BYTES;
+  __half *new_kv = reinterpret_cast<__half *>(ring + RING_BYTES);  // [K, V][HD]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
 
   // rows 0 .. G-1: the query heads of this kv head; the other rows of the tile are zero
-  for (int i = tid; i < 16 * (HD / 4); i += THREADS) {
-    const int r = i / (HD / 4), c4 = i - r * (HD / 4);
-    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (r < G) v = reinterpret_cast<const float4 *>(A.q + ((size_t)c * A.heads + (size_t)(kvh * G + r)) * HD)[c4];
-    uint2 hi, lo;
-    split2(v.x, v.y, hi.x, lo.x);
-    split2(v.z, v.w, hi.y, lo.y);
-    *reinterpret_cast<uint2 *>(q_hi + r * LD + 4 * c4) = hi;
-    *reinterpret_cast<uint2 *>(q_lo + r * LD + 4 * c4) = lo;
+  if constexpr (FUSED) {
+    // de-interleaved and rotated as rope_append does it, every product and sum rounded separately
+    const int qw = A.heads * HD, kw = A.kv_heads * HD;
+    const float *row = A.qkv + (size_t)c * (qw + 2 * kw);
+    const float *ct = A.cos_t + (size_t)pos * (HD / 2), *st = A.sin_t + (size_t)pos * (HD / 2);
+    for (int it = tid; it < (G + 1) * (HD / 2); it += THREADS) {  // row G: the new key
+      const int r = it / (HD / 2), i = it - r * (HD / 2);
+      if (r == G && !has_new) continue;
+      const float *src = row + (r < G ? (size_t)(kvh * G + r) * HD : (size_t)qw + (size_t)kvh * HD);
+      const float2 x = *reinterpret_cast<const float2 *>(src + 2 * i);
+      const float cs = ct[i], sn = st[i];
+      const float y1 = __fsub_rn(__fmul_rn(x.x, cs), __fmul_rn(x.y, sn)), y2 = __fadd_rn(__fmul_rn(x.y, cs), __fmul_rn(x.x, sn));
+      if (r < G) {
+        const __half h1 = __float2half_rn(y1), h2 = __float2half_rn(y2);
+        q_hi[r * LD + i] = h1;
+        q_hi[r * LD + HD / 2 + i] = h2;
+        q_lo[r * LD + i] = __float2half_rn(y1 - __half2float(h1));
+        q_lo[r * LD + HD / 2 + i] = __float2half_rn(y2 - __half2float(h2));
+      } else {
+        new_kv[i] = __float2half_rn(y1);
+        new_kv[HD / 2 + i] = __float2half_rn(y2);
+      }
+    }
+    if (has_new) new_kv[HD + tid] = __float2half_rn(row[qw + kw + (size_t)kvh * HD + tid]);
+    for (int i = tid; i < (16 - G) * (LD / 8); i += THREADS) {
+      reinterpret_cast<uint4 *>(q_hi + G * LD)[i] = make_uint4(0u, 0u, 0u, 0u);
+      reinterpret_cast<uint4 *>(q_lo + G * LD)[i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  } else {
+    for (int i = tid; i < 16 * (HD / 4); i += THREADS) {
+      const int r = i / (HD / 4), c4 = i - r * (HD / 4);
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (r < G) v = reinterpret_cast<const float4 *>(A.q + ((size_t)c * A.heads + (size_t)(kvh * G + r)) * HD)[c4];
+      uint2 hi, lo;
+      split2(v.x, v.y, hi.x, lo.x);
+      split2(v.z, v.w, hi.y, lo.y);
+      *reinterpret_cast<uint2 *>(q_hi + r * LD + 4 * c4) = hi;
+      *reinterpret_cast<uint2 *>(q_lo + r * LD + 4 * c4) = lo;
+    }
   }
   const __half *kc = static_cast<const __half *>(A.k_cache) + ((size_t)seq * A.kv_heads + kvh) * (size_t)A.ctx * HD;
   const __half *vc = static_cast<const __half *>(A.v_cache) + ((size_t)seq * A.kv_heads + kvh) * (size_t)A.ctx * HD;
@@ -119,13 +170,14 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_tc_kernel(const AttnAr
   const int n_tiles_cta = (p1 - p0 + TK - 1) / TK;
   const int n_my = n_tiles_cta > warp ? (n_tiles_cta - warp + WARPS - 1) / WARPS : 0;
   const uint32_t ring_s = smem_u32(ring) + (uint32_t)(warp * NSTG * STAGE_BYTES);
+  const int p_cached = has_new ? p1 - 1 : p1;  // the new row is not in the cache yet
   // a lane copies 16-byte piece (lane & 15) of keys (lane >> 4) + 2 r, r = 0..7, of K and of V
   auto issue = [&](int j) {
     if (j < n_my) {
       const int k0 = p0 + TK * (warp + WARPS * j);
       const int piece = lane & 15, key0 = lane >> 4;
       const uint32_t dst0 = ring_s + (uint32_t)((j % NSTG) * STAGE_BYTES) + (uint32_t)((key0 * LD + 8 * piece) * 2);
-      if (k0 + TK <= p1) {  // a whole tile: fixed offsets from one address per cache
+      if (k0 + TK <= p_cached) {  // a whole tile: fixed offsets from one address per cache
         const __half *ksrc = kc + (size_t)(k0 + key0) * HD + 8 * piece, *vsrc = vc + (size_t)(k0 + key0) * HD + 8 * piece;
 #pragma unroll
         for (int r = 0; r < TK / 2; ++r) {
@@ -136,8 +188,8 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_tc_kernel(const AttnAr
 #pragma unroll
         for (int r = 0; r < TK / 2; ++r) {
           const int key = key0 + 2 * r;
-          const bool live = k0 + key < p1;
-          const size_t src = (size_t)(live ? k0 + key : p1 - 1) * HD + 8 * piece;  // a valid address either way
+          const bool live = k0 + key < p_cached;
+          const size_t src = (size_t)(live ? k0 + key : p0) * HD + 8 * piece;  // a valid address either way
           cp_async16(dst0 + (uint32_t)(r * 2 * LD * 2), kc + src, live ? 16u : 0u);
           cp_async16(dst0 + (uint32_t)(r * 2 * LD * 2 + TK * LD * 2), vc + src, live ? 16u : 0u);
         }
@@ -147,7 +199,13 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_tc_kernel(const AttnAr
   };
   issue(0);
   issue(1);
-  __syncthreads();  // the query planes are in place
+  __syncthreads();  // the query planes (and the new row) are in place
+  if (has_new && tid < 2 * (HD / 8)) {  // append it
+    const int kv = tid / (HD / 8), piece = tid % (HD / 8);
+    __half *dst = (static_cast<__half *>(const_cast<void *>(kv ? A.v_cache : A.k_cache)) +
+                   (((size_t)seq * A.kv_heads + kvh) * (size_t)A.ctx + pos) * HD);
+    reinterpret_cast<uint4 *>(dst)[piece] = reinterpret_cast<const uint4 *>(new_kv + kv * HD)[piece];
+  }
 
   float m_run = -INFINITY, l_run = 0.0f;  // of row g (a query head when g < G)
   float o[HD / 8][4];
@@ -164,6 +222,12 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_tc_kernel(const AttnAr
     __syncwarp();        // ... and for every lane's
     const int k0 = p0 + TK * (warp + WARPS * j);
     const uint32_t ks_s = ring_s + (uint32_t)((j % NSTG) * STAGE_BYTES), vs_s = ks_s + TK * LD * 2;
+    if (has_new && pos - k0 < TK && pos >= k0) {  // this warp's tile holds the new position
+      __half *tile = reinterpret_cast<__half *>(ring + (size_t)warp * NSTG * STAGE_BYTES + (size_t)(j % NSTG) * STAGE_BYTES);
+      reinterpret_cast<uint4 *>(tile + ((lane >> 4) * TK + (pos - k0)) * LD)[lane & 15] =
+          reinterpret_cast<const uint4 *>(new_kv + (lane >> 4) * HD)[lane & 15];
+      __syncwarp();
+    }
     // ---- scores of 16 rows x 16 keys
     // (the two query planes accumulate separately: four independent chains of eight products)
     float s[2][4], sl[2][4];
@@ -270,12 +334,44 @@ __global__ void __launch_bounds__(THREADS, 2) attn_decode_tc_kernel(const AttnAr
       L = fmaf(ps[1], wgt, L);
       acc = fmaf(ps[2 + tid], wgt, acc);
     }
-    float *dst = A.scratch + (((size_t)c * A.heads + (size_t)(kvh * G + head)) * per_head + sp) * (HD + 2);
+    float *dst = FUSED ? mb + MERGE_FLOATS + head * (HD + 2)
+                       : A.scratch + (((size_t)c * A.heads + (size_t)(kvh * G + head)) * per_head + sp) * (HD + 2);
     dst[2 + tid] = acc;
     if (tid == 0) {
       dst[0] = M;
       dst[1] = L;
     }
+  }
+  if constexpr (FUSED) {
+    cluster_sync();
+    // spans of one head in span order, as in the second kernel; a CTA of the cluster takes every per_head-th head
+    for (int head = sp; head < G; head += per_head) {
+      const float *res = mb + MERGE_FLOATS + head * (HD + 2);
+      float ms[MAX_CLUSTER], ls[MAX_CLUSTER], vs[MAX_CLUSTER];
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s)
+        if (s < nspl) {
+          ms[s] = ld_cluster(res, s);
+          ls[s] = ld_cluster(res + 1, s);
+          vs[s] = ld_cluster(res + 2 + tid, s);
+        }
+      float M = -INFINITY, L = 0.0f, acc = 0.0f;
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s)
+        if (s < nspl) M = fmaxf(M, ms[s]);
+#pragma unroll
+      for (int s = 0; s < MAX_CLUSTER; ++s)
+        if (s < nspl) {
+          const float wgt = exp2f(__fmul_rn(__fsub_rn(ms[s], M), 1.44269504088896340736f));
+          L = fmaf(ls[s], wgt, L);
+          acc = fmaf(vs[s], wgt, acc);
+        }
+      const float v = __fmul_rn(acc, __frcp_rn(L));
+      const int k = (kvh * G + head) * HD + tid;
+      if (A.out_pack) xpack_store(static_cast<__half *>(A.out_pack), 2 * A.cols, c, k, v);
+      if (A.out_f32) A.out_f32[(size_t)c * A.heads * HD + k] = v;
+    }
+    cluster_sync();  // no CTA leaves while another may still read its result
   }
 }
 
@@ -304,9 +400,9 @@ __global__ void __launch_bounds__(HD) attn_decode_tc_combine_kernel(const float 
   if (out_f32) out_f32[(size_t)c * heads * HD + k] = v;
 }
 
-template <int G>
+template <int G, bool FUSED>
 cudaError_t launch_g(const AttnArgs &a, const LaunchCfg &cfg, int per_head) {
-  auto kernel = attn_decode_tc_kernel<G>;
+  auto kernel = attn_decode_tc_kernel<G, FUSED>;
   static DeviceOnce attr_once;  // per instantiation and device
   bool *attr_flag = attr_once.slot();
   if (!attr_flag || !*attr_flag) {
@@ -319,11 +415,21 @@ cudaError_t launch_g(const AttnArgs &a, const LaunchCfg &cfg, int per_head) {
   lc.blockDim = dim3(THREADS);
   lc.dynamicSmemBytes = SMEM_BYTES;
   lc.stream = cfg.stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (FUSED) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = (unsigned)per_head;
+    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (cfg.pdl) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
   lc.attrs = at;
-  lc.numAttrs = cfg.pdl ? 1 : 0;
+  lc.numAttrs = (unsigned)n;
   return cudaLaunchKernelEx(&lc, kernel, a, per_head);
 }
 
@@ -353,20 +459,34 @@ size_t attention_decode_tc_scratch_floats(int sm_count, int heads, int kv_heads,
   return (size_t)cols * heads * spans_per_head(sm_count, kv_heads, cols, ctx) * (HD + 2);
 }
 
+template <bool FUSED>
+static cudaError_t launch_spans(const AttnArgs &a, const LaunchCfg &cfg, int per_head) {
+  switch (a.heads / a.kv_heads) {
+    case 1: return launch_g<1, FUSED>(a, cfg, per_head);
+    case 2: return launch_g<2, FUSED>(a, cfg, per_head);
+    case 4: return launch_g<4, FUSED>(a, cfg, per_head);
+    default: return launch_g<8, FUSED>(a, cfg, per_head);
+  }
+}
+
+bool attention_decode_tc_fused(const AttnArgs &a, int sm_count) {
+  return attention_decode_tc_supported(a) && spans_per_head(sm_count, a.kv_heads, a.cols, a.ctx) <= MAX_CLUSTER;
+}
+
 cudaError_t launch_attention_decode_tc(const AttnArgs &a, const LaunchCfg &cfg) {
   count_launch(LC_ATTN_DECODE_TC);
+  if (a.qkv) {
+    const int sms = cfg.sm_count > 0 ? cfg.sm_count : 148;
+    if (!attention_decode_tc_fused(a, sms) || !a.cos_t || !a.sin_t || !a.k_cache || !a.v_cache || a.cols < 1 || (!a.out_pack && !a.out_f32))
+      return cudaErrorInvalidValue;
+    return launch_spans<true>(a, cfg, spans_per_head(sms, a.kv_heads, a.cols, a.ctx));
+  }
   if (!attention_decode_tc_supported(a) || !a.q || !a.k_cache || !a.v_cache || !a.scratch || a.cols < 1 ||
       (!a.out_pack && !a.out_f32))
     return cudaErrorInvalidValue;
   const int sms = cfg.sm_count > 0 ? cfg.sm_count : 148;
   const int per_head = spans_per_head(sms, a.kv_heads, a.cols, a.ctx);
-  cudaError_t e;
-  switch (a.heads / a.kv_heads) {
-    case 1: e = launch_g<1>(a, cfg, per_head); break;
-    case 2: e = launch_g<2>(a, cfg, per_head); break;
-    case 4: e = launch_g<4>(a, cfg, per_head); break;
-    default: e = launch_g<8>(a, cfg, per_head); break;
-  }
+  cudaError_t e = launch_spans<false>(a, cfg, per_head);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3((unsigned)a.heads, (unsigned)a.cols);

@@ -280,6 +280,9 @@ struct AttnArgs {
   float *scratch = nullptr;
   void *out_pack = nullptr;  // packed [K = heads*hd], batch = cols
   float *out_f32 = nullptr;  // optional plain copy [cols, heads*hd]
+  // launch_attention_decode_tc only: the raw projections [cols, qw + 2 * kw] and the rotation tables.  With them the launch rotates
+  // and appends itself (q is unused); attention_decode_tc_fused says whether it takes them.
+  const float *qkv = nullptr, *cos_t = nullptr, *sin_t = nullptr;
 };
 constexpr int ATTN_SPAN = 128;  // context positions per CTA of the split kernel
 bool attention_supported(int heads, int kv_heads, int hd);  // hd in {64,128}, heads/kv_heads in {1,2,4,8}
@@ -289,6 +292,7 @@ cudaError_t launch_attention(const AttnArgs &a, const LaunchCfg &cfg);
 // (attn_decode_tc.cu): per-warp cp.async rings keep the K / V stream going.  Two launches (spans, merge).
 bool attention_decode_tc_supported(const AttnArgs &a);
 size_t attention_decode_tc_scratch_floats(int sm_count, int heads, int kv_heads, int cols, int ctx);
+bool attention_decode_tc_fused(const AttnArgs &a, int sm_count);
 cudaError_t launch_attention_decode_tc(const AttnArgs &a, const LaunchCfg &cfg);
 
 // RoPE + KV append + split-context attention + combine in one launch (attn_fused.cu).  qkv rows are

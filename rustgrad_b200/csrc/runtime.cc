@@ -580,6 +580,15 @@ static bool decode_tc_attention(const rg_session *s, int ncols) {
              attn_scratch_floats(SCOLS, s->heads_l, s->cfg.head_dim, s->ctx);
 }
 
+// Rotation and cache append inside the tensor-core decode attention: plain layers, few enough spans for a cluster.
+static bool fuse_decode_tc(const rg_session *s, const RopeArgs &ra, AttnArgs *aa) {
+  if (s->variant || !attention_decode_tc_fused(*aa, s->sm_count)) return false;
+  aa->qkv = ra.qkv;
+  aa->cos_t = ra.cos_t;
+  aa->sin_t = ra.sin_t;
+  return true;
+}
+
 // True when every projection of the model can run the integer tensor-core GEMV at this width.
 static bool small_batch_path(const rg_session *s, int ncols) {
   if (ncols > 2 || s->opt.general_path_only || s->variant) return false;
@@ -1309,7 +1318,6 @@ static int32_t forward(rg_session *s, int ncols, int n_logit_cols, bool advance)
     ra.v_cache = s->v_cache[(size_t)l];
     ra.kv_f32 = s->kv_f32;
     rope_variant(s, W, &ra);
-    RG_LAUNCH(s, launch_rope_append(ra, L));
     AttnArgs aa;
     aa.q = s->q_rot;
     aa.k_cache = ra.k_cache;
@@ -1325,12 +1333,17 @@ static int32_t forward(rg_session *s, int ncols, int n_logit_cols, bool advance)
     aa.scratch = s->attn_scratch;
     aa.out_pack = s->attn_pack;
     aa.out_f32 = W.o.packed() ? nullptr : s->attn_f32;
-    if (tc_attn) {
+    if (tc_attn && fuse_decode_tc(s, ra, &aa)) {
       RG_LAUNCH(s, launch_attention_decode_tc(aa, L));
     } else {
-      RG_LAUNCH(s, launch_attention(aa, L));
+      RG_LAUNCH(s, launch_rope_append(ra, L));
+      if (tc_attn) {
+        RG_LAUNCH(s, launch_attention_decode_tc(aa, L));
+      } else {
+        RG_LAUNCH(s, launch_attention(aa, L));
+      }
+      if (s->family_mask & (1u << PROF_ATTN)) s->launches_in_step++;  // split + combine
     }
-    if (s->family_mask & (1u << PROF_ATTN)) s->launches_in_step++;  // split + combine
     }
     const DevTensor *ow[1] = {&W.o};
     if (s->tp_world > 1) {
