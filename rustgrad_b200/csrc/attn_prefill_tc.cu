@@ -56,6 +56,16 @@ __device__ __forceinline__ void split2(float x0, float x1, uint32_t &hi, uint32_
   lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+// 16 bytes global -> shared without a register stop; src_bytes = 0 writes zeros
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // f32 -> f16 as the GEMM operand conversion does it: finite values beyond the f16 range saturate
 __device__ __forceinline__ __half f16_sat(float v) {
   if (fabsf(v) > 65504.0f && fabsf(v) < __int_as_float(0x7f800000)) v = copysignf(65504.0f, v);
@@ -74,8 +84,9 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc_kernel(const PrefillA
   __half *vs = ks + TK * LD;                        // [TK][LD]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int kvh = blockIdx.y;
-  const int t0 = blockIdx.x * TQ;  // first query token of this CTA within the chunk
+  const int kvh = blockIdx.x;
+  // the CTAs with the most keys come first (all kv heads of them), so that the short ones fill the last wave
+  const int t0 = (int)(gridDim.y - 1 - blockIdx.y) * TQ;  // first query token of this CTA within the chunk
   if (t0 >= A.cols) return;
   const int nq = min(TQ, A.cols - t0);
   // row r = head * TQ + token  <->  query head kvh * G + head, token t0 + token; two f16 planes
@@ -111,19 +122,25 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc_kernel(const PrefillA
   const uint32_t vb_off = (uint32_t)((((lane & 7) + ((lane >> 3) & 1) * 8) * LD + (lane >> 4) * 8) * 2);              // B^T: two hd tiles
   const uint32_t qh_s = smem_u32(q_hi), ql_s = smem_u32(q_lo), ks_s = smem_u32(ks), vs_s = smem_u32(vs);
 
-  for (int k0 = 0; k0 <= last_q; k0 += TK) {
-    __syncthreads();  // the previous tile's K / V are no longer read (and Q is in place before the first tile)
-    for (int i = tid; i < TK * (HD / 8); i += THREADS) {  // 16-byte pieces; keys beyond the last visible position read as zero
-      const int key = i / (HD / 8), c = i - key * (HD / 8);
-      uint4 kq = make_uint4(0u, 0u, 0u, 0u), vq = kq;
-      if (k0 + key <= last_q) {
-        kq = *reinterpret_cast<const uint4 *>(kc + (size_t)(k0 + key) * HD + 8 * c);
-        vq = *reinterpret_cast<const uint4 *>(vc + (size_t)(k0 + key) * HD + 8 * c);
+  // One tile's 16-byte pieces to shared memory; keys beyond the last visible position arrive as zeros.  K of the next tile
+  // travels behind this tile's softmax and P V, V behind the next scores.  Loads that
+  // stopped in registers between two barriers, short CTAs first: 208 us a layer and chunk of a 2048-token prompt, now 162.  What is
+  // left is the tensor pipe (a scheduler takes 32 cycles for an m16n8k16).
+  auto copy = [&](const __half *src, uint32_t dst, int k0) {
+    if (k0 <= last_q) {
+      for (int i = tid; i < TK * (HD / 8); i += THREADS) {
+        const int key = i / (HD / 8), c = i - key * (HD / 8);
+        const bool live = k0 + key <= last_q;
+        cp_async16(dst + (uint32_t)((key * LD + 8 * c) * 2), src + (size_t)(live ? k0 + key : last_q) * HD + 8 * c, live ? 16u : 0u);
       }
-      *reinterpret_cast<uint4 *>(ks + key * LD + 8 * c) = kq;
-      *reinterpret_cast<uint4 *>(vs + key * LD + 8 * c) = vq;
     }
-    __syncthreads();
+    cp_async_commit();  // an empty group keeps the count of groups in flight uniform
+  };
+  copy(kc, ks_s, 0);
+  copy(vc, vs_s, 0);
+  for (int k0 = 0; k0 <= last_q; k0 += TK) {
+    cp_async_wait<1>();  // K has landed, V may be under way
+    __syncthreads();     // ... every thread's pieces (and Q is in place before the first tile)
     // ---- scores of 16 rows x 64 keys
     float s[TK / 8][4];
 #pragma unroll
@@ -143,6 +160,8 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc_kernel(const PrefillA
         mma_f16(s[2 * n2 + 1], ah, b[2], b[3]);
       }
     }
+    __syncthreads();  // K is no longer read
+    copy(kc, ks_s, k0 + TK);
     // ---- scale, mask, online softmax: the four lanes of a quad share a row
     float corr[2];
 #pragma unroll
@@ -188,6 +207,8 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc_kernel(const PrefillA
       o[n][2] *= corr[1];
       o[n][3] *= corr[1];
     }
+    cp_async_wait<1>();  // V has landed
+    __syncthreads();
     // ---- O += P V: two adjacent 8-key score tiles are one 16-key A fragment
 #pragma unroll
     for (int kt = 0; kt < TK / 16; ++kt) {
@@ -206,7 +227,10 @@ __global__ void __launch_bounds__(THREADS) attn_prefill_tc_kernel(const PrefillA
         mma_f16(o[2 * n2 + 1], ph, b[2], b[3]);
       }
     }
+    __syncthreads();  // V is no longer read
+    copy(vc, vs_s, k0 + TK);
   }
+  cp_async_wait<0>();
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int r = 16 * warp + g + 8 * h, head = r / TQ, tok = r - head * TQ;
@@ -253,7 +277,7 @@ cudaError_t launch_t(const PrefillAttnArgs &a, const LaunchCfg &cfg) {
   }
   constexpr int TQ = ROWS / G;
   cudaLaunchConfig_t lc{};
-  lc.gridDim = dim3((unsigned)((a.cols + TQ - 1) / TQ), (unsigned)a.kv_heads);
+  lc.gridDim = dim3((unsigned)a.kv_heads, (unsigned)((a.cols + TQ - 1) / TQ));
   lc.blockDim = dim3(THREADS);
   lc.dynamicSmemBytes = smem;
   lc.stream = cfg.stream;
