@@ -1,0 +1,208 @@
+// Copies between pageable host arrays and the device for the operator entry points.
+//
+// A copy from or to pageable memory goes through a small staging buffer of the driver on the calling thread, at a
+// fraction of the bus rate, and a fresh result array takes its page faults on that thread too.  Here four threads fill (or
+// empty) pinned pieces of 1 MB while others are on the bus, so the bus, the page faults and the look at the block scales run side
+// by side.  rg_b200_qgemm Q4_0 [14336, 4096] x 512 (33 + 8 MB up, 29 MB down) 10.8 -> 4.1 ms, rg_b200_qmatmul Q8_0 [4096, 4096] x 4
+// (18 MB up) 3.6 -> 1.35 ms; the bus alone takes about 1.4 and 0.4.
+#include "host_copy.h"
+
+#include <string.h>
+
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+#include <new>
+#include <system_error>
+#include <thread>
+
+namespace rg {
+
+struct HostStaging {
+  int device = -1;
+  cudaStream_t stream = nullptr;
+  uint8_t *pinned = nullptr;  // PIECES pieces
+  cudaEvent_t done[HostCall::PIECES] = {};
+  ~HostStaging() {
+    for (cudaEvent_t e : done)
+      if (e) cudaEventDestroy(e);
+    if (stream) cudaStreamDestroy(stream);
+    if (pinned) cudaFreeHost(pinned);
+  }
+};
+
+namespace {
+
+std::mutex g_mutex;
+HostStaging *g_idle[HostCall::IDLE_KEEP] = {};
+int g_n_idle = 0;
+cudaMemPool_t g_pools[64] = {};
+
+cudaError_t pool_of(int device, cudaMemPool_t *out) {
+  if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  if (!g_pools[device]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = HostCall::POOL_KEEP;
+    if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    g_pools[device] = pool;
+  }
+  *out = g_pools[device];
+  return cudaSuccess;
+}
+
+// Runs work(t) for t < n on as many threads as can be started, the caller's among them.
+template <typename F>
+void on_threads(int n, F work) {
+  std::thread extra[HostCall::THREADS];
+  int started = 0;
+  std::atomic<int> next{0};
+  auto body = [&] {
+    for (int t; (t = next.fetch_add(1)) < n;) work(t);
+  };
+  try {
+    for (; started < n - 1; ++started) extra[started] = std::thread(body);
+  } catch (...) {  // no more threads: the ones there are share the work
+  }
+  body();
+  for (int i = 0; i < started; ++i) extra[i].join();
+}
+
+}  // namespace
+
+HostCall::~HostCall() {
+  if (!st_) return;
+  cudaStreamSynchronize(st_->stream);  // nothing of this call is left in flight, whatever it returned
+  for (int i = 0; i < n_bufs_; ++i) cudaFreeAsync(bufs_[i], st_->stream);
+  cudaStreamSynchronize(st_->stream);  // the pool gives back what it holds above POOL_KEEP
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (g_n_idle < IDLE_KEEP) {
+      g_idle[g_n_idle++] = st_;
+      st_ = nullptr;
+    }
+  }
+  delete st_;
+}
+
+cudaStream_t HostCall::stream() const { return st_->stream; }
+
+cudaError_t HostCall::open(int device) {
+  device_ = device;
+  cudaError_t e = cudaSetDevice(device);
+  if (e != cudaSuccess) return e;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    for (int i = 0; i < g_n_idle; ++i)
+      if (g_idle[i]->device == device) {
+        st_ = g_idle[i];
+        g_idle[i] = g_idle[--g_n_idle];
+        return cudaSuccess;
+      }
+  }
+  HostStaging *st = new (std::nothrow) HostStaging;
+  if (!st) return cudaErrorMemoryAllocation;
+  st->device = device;
+  e = cudaStreamCreateWithFlags(&st->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&st->pinned), PIECES * PIECE, cudaHostAllocDefault);
+  for (cudaEvent_t &ev : st->done)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    delete st;
+    return e;
+  }
+  st_ = st;
+  return cudaSuccess;
+}
+
+cudaError_t HostCall::alloc_bytes(void **p, size_t bytes) {
+  cudaMemPool_t pool;
+  cudaError_t e = pool_of(device_, &pool);
+  if (e != cudaSuccess) return e;
+  if (n_bufs_ == MAX_BUFFERS) return cudaErrorInvalidValue;
+  if ((e = cudaMallocFromPoolAsync(p, bytes, pool, st_->stream)) != cudaSuccess) return e;
+  bufs_[n_bufs_++] = *p;
+  return cudaSuccess;
+}
+
+cudaError_t HostCall::upload(void *dst, const void *src, size_t bytes, size_t block, bool (*bad)(const uint8_t *), int64_t *first_bad) {
+  const size_t piece = block ? PIECE / block * block : PIECE, pieces = (bytes + piece - 1) / piece;
+  std::atomic<int64_t> lowest{INT64_MAX};
+  std::atomic<int> error{cudaSuccess};
+  HostStaging *st = st_;
+  const int threads = (int)std::min<size_t>(THREADS, pieces);
+  auto work = [&](int t) {
+    if (cudaSetDevice(st->device) != cudaSuccess) {
+      error = cudaErrorInvalidDevice;
+      return;
+    }
+    int use = 0;
+    for (size_t i = (size_t)t; i < pieces && error == cudaSuccess; i += (size_t)threads, ++use) {
+      const int slot = 2 * t + (use & 1);
+      const size_t at = i * piece, n = std::min(piece, bytes - at);
+      const uint8_t *from = static_cast<const uint8_t *>(src) + at;
+      cudaError_t e = cudaEventSynchronize(st->done[slot]);  // an event not yet recorded is over
+      if (e == cudaSuccess) {
+        if (bad)
+          for (size_t b = 0; b + block <= n; b += block)
+            if (bad(from + b)) {
+              const int64_t at_block = (int64_t)((at + b) / block);
+              int64_t seen = lowest.load();
+              while (at_block < seen && !lowest.compare_exchange_weak(seen, at_block)) {
+              }
+              break;
+            }
+        memcpy(st->pinned + (size_t)slot * PIECE, from, n);
+        e = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + at, st->pinned + (size_t)slot * PIECE, n, cudaMemcpyHostToDevice, st->stream);
+      }
+      if (e == cudaSuccess) e = cudaEventRecord(st->done[slot], st->stream);
+      if (e != cudaSuccess) error = e;
+    }
+  };
+  on_threads(threads, work);
+  if (first_bad) *first_bad = lowest == INT64_MAX ? -1 : lowest.load();
+  return (cudaError_t)error.load();
+}
+
+cudaError_t HostCall::download(void *dst, const void *src, size_t bytes) {
+  const size_t pieces = (bytes + PIECE - 1) / PIECE;
+  std::atomic<int> error{cudaSuccess};
+  HostStaging *st = st_;
+  const int threads = (int)std::min<size_t>(THREADS, pieces);
+  auto work = [&](int t) {
+    if (cudaSetDevice(st->device) != cudaSuccess) {
+      error = cudaErrorInvalidDevice;
+      return;
+    }
+    auto ask = [&](size_t i, int slot) {
+      if (i >= pieces) return cudaSuccess;
+      cudaError_t e = cudaMemcpyAsync(st->pinned + (size_t)slot * PIECE, static_cast<const uint8_t *>(src) + i * PIECE,
+                                      std::min(PIECE, bytes - i * PIECE), cudaMemcpyDeviceToHost, st->stream);
+      return e == cudaSuccess ? cudaEventRecord(st->done[slot], st->stream) : e;
+    };
+    // the slots' last uploads lie in front of these copies on the stream
+    cudaError_t e = ask((size_t)t, 2 * t);
+    int use = 0;
+    for (size_t i = (size_t)t; i < pieces && e == cudaSuccess; i += (size_t)threads, ++use) {
+      const int slot = 2 * t + (use & 1);
+      e = ask(i + (size_t)threads, slot ^ 1);
+      if (e == cudaSuccess) e = cudaEventSynchronize(st->done[slot]);
+      if (e == cudaSuccess) memcpy(static_cast<uint8_t *>(dst) + i * PIECE, st->pinned + (size_t)slot * PIECE, std::min(PIECE, bytes - i * PIECE));
+    }
+    if (e != cudaSuccess) error = e;
+  };
+  on_threads(threads, work);
+  return (cudaError_t)error.load();
+}
+
+}  // namespace rg

@@ -1,0 +1,54 @@
+// Device buffers, a stream and pinned staging for one operator call on host arrays, kept between calls.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stddef.h>
+#include <stdint.h>
+
+namespace rg {
+
+struct HostStaging;  // a stream, its pinned pieces and their events
+
+// One operator call.  Device buffers come from a private memory pool of the device (at most POOL_KEEP bytes stay with
+// it when nothing is in use), stream and pinned pieces from a list of at most IDLE_KEEP idle sets per process; all of
+// it goes back when the call ends, on every path, after its work on the stream is over.  Calls on different threads
+// use different sets.
+class HostCall {
+ public:
+  static constexpr size_t PIECE = size_t(1) << 20;  // bytes of a pinned piece
+  static constexpr int THREADS = 4;                 // host threads that copy a large array
+  static constexpr int PIECES = 2 * THREADS;        // two of a thread: one is filled while the other is on the bus
+  static constexpr size_t POOL_KEEP = size_t(256) << 20;
+  static constexpr int IDLE_KEEP = 4;
+  static constexpr int MAX_BUFFERS = 8;             // device buffers of one call
+
+  HostCall() = default;
+  ~HostCall();
+  HostCall(const HostCall &) = delete;
+  HostCall &operator=(const HostCall &) = delete;
+
+  cudaError_t open(int device);
+  cudaStream_t stream() const;
+  template <typename T>
+  cudaError_t alloc(T **p, size_t bytes) {
+    void *raw = nullptr;
+    const cudaError_t e = alloc_bytes(&raw, bytes ? bytes : 16);
+    *p = static_cast<T *>(raw);
+    return e;
+  }
+  // Host -> device on the stream; src may be reused when the call returns.  `bad` (nullable) looks at every whole `block`-byte block
+  // on the way and returns true for one that is refused; *first_bad is the lowest such block or -1.
+  cudaError_t upload(void *dst, const void *src, size_t bytes, size_t block = 0, bool (*bad)(const uint8_t *) = nullptr,
+                     int64_t *first_bad = nullptr);
+  // Device -> host behind the work of the stream; dst is complete when the call returns.
+  cudaError_t download(void *dst, const void *src, size_t bytes);
+
+ private:
+  cudaError_t alloc_bytes(void **p, size_t bytes);
+  int device_ = -1;
+  HostStaging *st_ = nullptr;
+  void *bufs_[MAX_BUFFERS] = {};
+  int n_bufs_ = 0;
+};
+
+}  // namespace rg

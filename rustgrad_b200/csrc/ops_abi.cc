@@ -10,6 +10,7 @@
 
 #include "../../include/rg_b200.h"
 #include "gguf.h"
+#include "host_copy.h"
 #include "kernels.h"
 
 #include <atomic>
@@ -132,6 +133,56 @@ int32_t scan_scales(int32_t type, const uint8_t *bytes, size_t nbytes) {
   return RG_OK;
 }
 
+// A Q4_0 / Q8_0 block whose scale is not finite.
+bool bad_scale(const uint8_t *block) { return ((block[1] >> 2) & 0x1f) == 0x1f; }
+
+// Opens a call on host arrays and brings weight and activation rows over.  The scales of packed weights are looked at on the
+// way; a weight that is refused for one is refused for it whatever else went wrong, as when the scan came first.
+int32_t open_call(HostCall *hc, LaunchCfg *cfg, int32_t device, int32_t type, const uint8_t *weight, size_t wbytes, const float *x,
+                  size_t xbytes, uint8_t **d_w, float **d_x, float **d_y, size_t ybytes, int **d_status) {
+  const auto go = [&]() -> int32_t {
+    OP_CUDA(hc->open(device));
+    int sms = 148;
+    OP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    OP_CUDA(hc->alloc(d_status, sizeof(int)));
+    OP_CUDA(hc->alloc(d_w, wbytes));
+    OP_CUDA(hc->alloc(d_x, xbytes));
+    OP_CUDA(hc->alloc(d_y, ybytes));
+    OP_CUDA(cudaMemsetAsync(*d_status, 0, sizeof(int), hc->stream()));
+    cfg->stream = hc->stream();
+    cfg->pdl = false;
+    cfg->sm_count = sms;
+    cfg->status = *d_status;
+    if (type == RG_TYPE_Q4_0 || type == RG_TYPE_Q8_0) {
+      int64_t first_bad = -1;
+      OP_CUDA(hc->upload(*d_w, weight, wbytes, (size_t)block_bytes(type), bad_scale, &first_bad));
+      if (first_bad >= 0) return fail(RG_NON_FINITE_SCALE, "block " + std::to_string(first_bad));
+    } else {
+      const int32_t rc = scan_scales(type, weight, wbytes);
+      if (rc) return rc;
+      OP_CUDA(hc->upload(*d_w, weight, wbytes));
+    }
+    OP_CUDA(hc->upload(*d_x, x, xbytes));
+    return RG_OK;
+  };
+  const int32_t rc = go();
+  if (rc == RG_OK || rc == RG_NON_FINITE_SCALE) return rc;
+  const std::string why = g_last_error;
+  const int32_t scanned = scan_scales(type, weight, wbytes);
+  return scanned ? scanned : fail(rc, why);
+}
+
+// Reads the result and the status word back; d_y's kernels are on the call's stream.
+int32_t close_call(HostCall *hc, const int *d_status, float *out, const float *d_y, size_t ybytes) {
+  int status = 0;
+  OP_CUDA(hc->download(out, d_y, ybytes));
+  OP_CUDA(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, hc->stream()));
+  OP_CUDA(cudaStreamSynchronize(hc->stream()));
+  if (status == 1) return fail(RG_TIMEOUT, "a bounded device-side wait gave up");
+  if (status) return fail(RG_CUDA_ERROR, "device status " + std::to_string(status));
+  return RG_OK;
+}
+
 // Workspace of the K-split row GEMV (qgemv_rows.cu): partial tiles and zeroed arrival counters.
 struct GemvWorkspace {
   float *scratch = nullptr;
@@ -139,12 +190,14 @@ struct GemvWorkspace {
   unsigned *counters = nullptr;
 };
 constexpr size_t GEMV_WS_FLOATS = (size_t)256 * 512 * 8;  // up to 256 units of 512 threads x 8 partial sums
-cudaError_t alloc_gemv_workspace(Scope *sc, GemvWorkspace *ws) {
+template <typename S>
+cudaError_t alloc_gemv_workspace(S *sc, cudaStream_t stream, GemvWorkspace *ws) {
+  if (!qgemv_rows_enabled()) return cudaSuccess;  // the other kernels need none
   cudaError_t e = sc->alloc(&ws->scratch, sizeof(float) * GEMV_WS_FLOATS);
   if (e != cudaSuccess) return e;
   if ((e = sc->alloc(&ws->counters, sizeof(unsigned) * QGEMV_ROWS_MAX_TILES)) != cudaSuccess) return e;
   ws->floats = GEMV_WS_FLOATS;
-  return cudaMemsetAsync(ws->counters, 0, sizeof(unsigned) * QGEMV_ROWS_MAX_TILES, sc->stream);
+  return cudaMemsetAsync(ws->counters, 0, sizeof(unsigned) * QGEMV_ROWS_MAX_TILES, stream);
 }
 
 // Activation rows one launch takes: 16 for the packed types (the f16-MMA GEMV), else 8.
@@ -249,29 +302,19 @@ int32_t rg_b200_qmatmul(int32_t device, int32_t type, const uint8_t *weight, uin
     return RG_OK;
   }
   if (packed && k % 256) return fail(RG_UNSUPPORTED_GEOMETRY, "packed weights need K to be a multiple of 256");
-  if ((rc = scan_scales(type, weight, wbytes))) return rc;
-  Scope sc;
+  HostCall hc;
   LaunchCfg cfg;
   int *d_status;
-  if ((rc = open_scope(device, &sc, &cfg, &d_status))) return rc;
   uint8_t *d_w, *d_pack;
   float *d_x, *d_y;
-  OP_CUDA(sc.alloc(&d_w, wbytes));
-  OP_CUDA(sc.alloc(&d_x, sizeof(float) * m * k));
-  OP_CUDA(sc.alloc(&d_y, sizeof(float) * m * n));
-  OP_CUDA(sc.alloc(&d_pack, xpack_bytes((int)k, 16)));
+  const size_t ybytes = sizeof(float) * m * n;
+  if ((rc = open_call(&hc, &cfg, device, type, weight, wbytes, activation, sizeof(float) * m * k, &d_w, &d_x, &d_y, ybytes, &d_status)))
+    return rc;
+  OP_CUDA(hc.alloc(&d_pack, xpack_bytes((int)k, 16)));
   GemvWorkspace ws;
-  OP_CUDA(alloc_gemv_workspace(&sc, &ws));
-  OP_CUDA(cudaMemcpyAsync(d_w, weight, wbytes, cudaMemcpyHostToDevice, sc.stream));
-  OP_CUDA(cudaMemcpyAsync(d_x, activation, sizeof(float) * m * k, cudaMemcpyHostToDevice, sc.stream));
+  OP_CUDA(alloc_gemv_workspace(&hc, hc.stream(), &ws));
   if ((rc = run_matmul(type, d_w, n, k, d_x, m, d_y, d_pack, ws, cfg))) return rc;
-  int status = 0;
-  OP_CUDA(cudaMemcpyAsync(out, d_y, sizeof(float) * m * n, cudaMemcpyDeviceToHost, sc.stream));
-  OP_CUDA(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, sc.stream));
-  OP_CUDA(cudaStreamSynchronize(sc.stream));
-  if (status == 1) return fail(RG_TIMEOUT, "a bounded device-side wait gave up");
-  if (status) return fail(RG_CUDA_ERROR, "device status " + std::to_string(status));
-  return RG_OK;
+  return close_call(&hc, d_status, out, d_y, ybytes);
 }
 
 int32_t rg_b200_row_gather(int32_t device, int32_t type, const uint8_t *weight, uint64_t rows, uint64_t cols,
@@ -315,20 +358,19 @@ int32_t rg_b200_qgemm(int32_t device, int32_t type, const uint8_t *weight, uint6
   if (rc) return rc;
   if (n == 0 || m == 0) return RG_OK;
   if (k == 0 || k % 256) return fail(RG_UNSUPPORTED_GEOMETRY, "packed weights need K to be a multiple of 256");
-  if ((rc = scan_scales(type, weight, wbytes))) return rc;
-  Scope sc;
+  if (operand_mode < 0 || operand_mode > 2) {
+    if ((rc = scan_scales(type, weight, wbytes))) return rc;
+    return fail(RG_INVALID_ARGUMENT, "operand_mode must be 0, 1 or 2");
+  }
+  HostCall hc;
   LaunchCfg cfg;
   int *d_status;
-  if ((rc = open_scope(device, &sc, &cfg, &d_status))) return rc;
   uint8_t *d_w, *d_xb;
   float *d_x, *d_y;
-  OP_CUDA(sc.alloc(&d_w, wbytes));
-  OP_CUDA(sc.alloc(&d_x, sizeof(float) * m * k));
-  if (operand_mode < 0 || operand_mode > 2) return fail(RG_INVALID_ARGUMENT, "operand_mode must be 0, 1 or 2");
-  OP_CUDA(sc.alloc(&d_xb, 4 * m * k));  // hi and lo planes
-  OP_CUDA(sc.alloc(&d_y, sizeof(float) * m * n));
-  OP_CUDA(cudaMemcpyAsync(d_w, weight, wbytes, cudaMemcpyHostToDevice, sc.stream));
-  OP_CUDA(cudaMemcpyAsync(d_x, activation, sizeof(float) * m * k, cudaMemcpyHostToDevice, sc.stream));
+  const size_t ybytes = sizeof(float) * m * n;
+  if ((rc = open_call(&hc, &cfg, device, type, weight, wbytes, activation, sizeof(float) * m * k, &d_w, &d_x, &d_y, ybytes, &d_status)))
+    return rc;
+  OP_CUDA(hc.alloc(&d_xb, 4 * m * k));  // hi and lo planes
   Operand16 op;
   op.hi = d_xb;
   op.lo = operand_mode == QGEMM_F16X3 ? d_xb + 2 * m * k : nullptr;
@@ -349,22 +391,25 @@ int32_t rg_b200_qgemm(int32_t device, int32_t type, const uint8_t *weight, uint6
   a.ldc = (int)n;
   OP_CUDA(launch_qgemm_tc(a, cfg));  // first launch also serves as warm-up
   const int reps = iters > 0 ? iters : 0;
-  OP_CUDA(cudaEventCreate(&sc.e0));
-  OP_CUDA(cudaEventCreate(&sc.e1));
-  OP_CUDA(cudaEventRecord(sc.e0, sc.stream));
-  for (int i = 0; i < reps; ++i) OP_CUDA(launch_qgemm_tc(a, cfg));
-  OP_CUDA(cudaEventRecord(sc.e1, sc.stream));
-  int status = 0;
-  OP_CUDA(cudaMemcpyAsync(out, d_y, sizeof(float) * m * n, cudaMemcpyDeviceToHost, sc.stream));
-  OP_CUDA(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, sc.stream));
-  OP_CUDA(cudaStreamSynchronize(sc.stream));
-  if (status == 1) return fail(RG_TIMEOUT, "a bounded device-side wait gave up");
-  if (status) return fail(RG_CUDA_ERROR, "device status " + std::to_string(status));
-  if (kernel_ms) {
-    float ms = 0.0f;
-    OP_CUDA(cudaEventElapsedTime(&ms, sc.e0, sc.e1));
-    *kernel_ms = reps ? ms / (float)reps : 0.0f;
+  float ms = 0.0f;
+  if (reps) {
+    struct Events {
+      cudaEvent_t e0 = nullptr, e1 = nullptr;
+      ~Events() {
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+      }
+    } ev;
+    OP_CUDA(cudaEventCreate(&ev.e0));
+    OP_CUDA(cudaEventCreate(&ev.e1));
+    OP_CUDA(cudaEventRecord(ev.e0, cfg.stream));
+    for (int i = 0; i < reps; ++i) OP_CUDA(launch_qgemm_tc(a, cfg));
+    OP_CUDA(cudaEventRecord(ev.e1, cfg.stream));
+    OP_CUDA(cudaEventSynchronize(ev.e1));
+    OP_CUDA(cudaEventElapsedTime(&ms, ev.e0, ev.e1));
   }
+  if ((rc = close_call(&hc, d_status, out, d_y, ybytes))) return rc;
+  if (kernel_ms) *kernel_ms = reps ? ms / (float)reps : 0.0f;
   return RG_OK;
 }
 
@@ -458,7 +503,7 @@ int32_t rg_b200_qmatmul_bench(int32_t device, int32_t type, const uint8_t *weigh
   a.y = d_y;
   a.ldy = (int)n;
   GemvWorkspace ws;
-  OP_CUDA(alloc_gemv_workspace(&sc, &ws));
+  OP_CUDA(alloc_gemv_workspace(&sc, sc.stream, &ws));
   a.split_scratch = ws.scratch;
   a.split_scratch_floats = ws.floats;
   a.split_counters = ws.counters;
