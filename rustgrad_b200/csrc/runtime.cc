@@ -1285,9 +1285,10 @@ static int32_t forward(rg_session *s, int ncols, int n_logit_cols, bool advance)
     if (rc) return rc;
     prof_mark(s, PROF_ATTN);
     const bool tc_attn = decode_tc_attention(s, ncols);
-    if (!tc_attn && (gemv16 || (ncols >= 3 && !s->chunk_is_prompt && !env_flag("RG_B200_SPLIT_ATTENTION_SMALL"))) &&
+    if (!tc_attn && (gemv16 || (!s->chunk_is_prompt && !env_flag("RG_B200_SPLIT_ATTENTION_SMALL"))) &&
         s->attn_counters && !s->variant) {
-      // rows of distinct sequences: RoPE, cache append, split attention and the combine in one launch
+      // rows of distinct sequences: RoPE, cache append, split attention and the combine in one launch (one row of a small f32
+      // model too: 8.7 us against 12.0 in three)
       FusedAttnArgs fa;
       fa.qkv = s->qkv;
       fa.cols = ncols;
