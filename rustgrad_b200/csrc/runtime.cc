@@ -2325,10 +2325,10 @@ int32_t rg_b200_prefill_rows(rg_session *s, const int32_t *rows, const int32_t *
 }
 
 // More than 16 decode rows on packed weights: such a step is cut into equal chunks of at most 16 rows for the 16-row
-// kernels (GEMV with four column tiles, tensor-core decode attention).  The rule was set when two half-size steps were
-// faster than one step on the 17..32-row path (8B shape, 32 rows: 3.8 against 3.1 thousand tokens/s).  Since the GEMM
-// there issues faster that no longer holds: 32 rows behind 512 positions take 8.0 ms in two passes and 6.5 in one, 17
-// rows 6.7 and 6.1, behind 2048 positions 9.3 and 7.7, 7.4 and 6.7.  The rows are independent sequences and positions
+// kernels (GEMV with up to four column tiles, tensor-core decode attention).  One step on the 17..32-row path is faster (8B shape, 32
+// rows behind 512 positions 7.3 ms in two passes and 5.3 in one, 17 rows 5.8 and 4.8; behind 2048 positions 9.1 and 7.1, 7.6 and
+// 5.9), but its tcgen05 products accumulate all of K in the tensor core: 1.4e-5 from 64 bits at K = 4096 and 4.8e-5 at 14336,
+// where the GEMV's per-block sums are 1.1e-7 and 1.4e-7 away.  The rows are independent sequences and positions
 // move only when every chunk has succeeded.
 static int decode_chunk_rows(const rg_session *s, int n) {
   if (n <= 16 || !s->packed_layers || env_flag("RG_B200_WIDE_DECODE_ONE_STEP")) return n;
