@@ -255,3 +255,36 @@ print("ok")
     env = dict(os.environ, RG_B200_ROWS_GEMV="1", PYTHONPATH=root + os.pathsep + os.environ.get("PYTHONPATH", ""))
     r = subprocess.run([sys.executable, "-c", code], env=env, cwd=root, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "ok" in r.stdout, r.stdout + r.stderr
+
+
+def test_operator_calls_move_large_arrays_in_pieces():
+    """Weights, activations and results of several 1 MB pieces: the lowest of two refused blocks is named wherever its piece lies, the call
+    after a refusal is whole, and calls on several threads do not meet."""
+    import threading
+    n, k, m = 2500, 2048, 130
+    rng = np.random.default_rng(3)
+    data = quant.encode(quant.Q8_0, (rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    bad = data.reshape(-1, quant.BLOCK_BYTES[quant.Q8_0]).copy()
+    for block in (159_999, 70_001):
+        bad[block, :2] = (0x00, 0x7C)  # an infinite scale
+    x = rng.standard_normal((m, k), dtype=np.float32)
+    for call in (session.qmatmul, session.qgemm):
+        with pytest.raises(session.RgError, match="block 70001"):
+            call(quant.Q8_0, bad.reshape(-1), n, k, x)
+    want = session.qmatmul(quant.Q8_0, data, n, k, x)
+    dense = O.dequantize(quant.Q8_0, data, n * k).reshape(n, k).astype(np.float64)
+    scale = np.sqrt((x.astype(np.float64) ** 2).sum(1))[:, None] * np.sqrt((dense ** 2).sum(1))[None, :]
+    assert (np.abs(want - x.astype(np.float64) @ dense.T) / scale).max() < 1e-6
+    got = [None] * 6
+
+    def one(i):
+        got[i] = session.qmatmul(quant.Q8_0, data, n, k, x[: m - i])
+
+    threads = [threading.Thread(target=one, args=(i,)) for i in range(len(got))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i, g in enumerate(got):
+        full = (m - i) // 16 * 16  # rows in chunks of sixteen like those of the whole call
+        np.testing.assert_array_equal(g[:full], want[:full])
